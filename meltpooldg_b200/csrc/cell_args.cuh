@@ -32,6 +32,7 @@ struct GeoParams {
   T detJ;                   // uniform box: det(J)
   T Gd[3];                  // uniform box: det(J) / h_d^2
   const T *__restrict__ q;  // deformed: [cell][7][n^3] = JxW, Gxx Gxy Gxz Gyy Gyz Gzz
+  const double *__restrict__ vert;  // deformed: the mesh's vertices, x fastest, 3 coordinates each
 };
 
 // Scalars of a device-resident Krylov iteration (read by kernels, finalised

@@ -29,8 +29,9 @@ enum MatKind { kS = 0, kST = 1, kD = 2, kDT = 3, kPT = 4, kQT = 5, kRT = 6, kNum
 
 MPDG_HD constexpr int kind_sym(int kind) { return (kind == kD || kind == kDT || kind == kRT) ? -1 : 1; }
 
-// Per (n, kind) block: ae[n][h], ao[n][h], mid[n] with h = n/2.
-MPDG_HD constexpr int tab_block(int n) { return 2 * n * (n / 2) + n; }
+// Per (n, kind) block: ae[n][h], ao[n][h], mid[n] with h = n/2, then the matrix itself [n][n].
+MPDG_HD constexpr int tab_full(int n) { return 2 * n * (n / 2) + n; }
+MPDG_HD constexpr int tab_block(int n) { return tab_full(n) + n * n; }
 MPDG_HD constexpr int tab_offset_n(int n)
 {
   int off = 0;
@@ -47,6 +48,9 @@ MPDG_HD constexpr int w_off(int n)
   return off;
 }
 constexpr int kWSize = w_off(kMaxN + 1);
+// the kernels' table of both: the Gauss weights of every n, then the Gauss points
+MPDG_HD constexpr int xg_off(int n) { return kWSize + w_off(n); }
+constexpr int kWTabSize = 2 * kWSize;
 
 struct Tables1D {
   int n = 0;
@@ -166,12 +170,12 @@ inline Tables1D make_tables(int n)
   return t;
 }
 
-// Flattened even-odd tables for all n = 2..kMaxN (what the kernels read).
+// Flattened even-odd and full tables for all n = 2..kMaxN (what the kernels read).
 inline void fill_even_odd(std::vector<double> &tab, std::vector<double> &w,
                           std::vector<double> &xl)
 {
   tab.assign(kTabSize, 0.0);
-  w.assign(kWSize, 0.0);
+  w.assign(kWTabSize, 0.0);
   xl.assign(kWSize, 0.0);
   for (int n = 2; n <= kMaxN; ++n) {
     const Tables1D t = make_tables(n);
@@ -184,10 +188,12 @@ inline void fill_even_odd(std::vector<double> &tab, std::vector<double> &w,
           blk[n * h + o * h + l] = 0.5 * (t.A[kind][o][l] - t.A[kind][o][n - 1 - l]);
         }
         blk[2 * n * h + o] = (n & 1) ? t.A[kind][o][h] : 0.0;
+        for (int l = 0; l < n; ++l) blk[tab_full(n) + o * n + l] = t.A[kind][o][l];
       }
     }
     for (int i = 0; i < n; ++i) {
       w[w_off(n) + i] = t.wg[i];
+      w[xg_off(n) + i] = t.xg[i];
       xl[w_off(n) + i] = t.xl[i];
     }
   }

@@ -1284,6 +1284,7 @@ static CellArgs<T> cell_args(mpdg_heat *h)
   a.g.detJ = (T)detJ;
   for (int e = 0; e < 3; ++e) a.g.Gd[e] = (T)(detJ / (h->hcell[e] * h->hcell[e]));
   a.g.q = nullptr;
+  a.g.vert = h->vert;
   const mpdg_material &m = h->mat;
   a.m.rho_l = (T)m.rho_l;
   a.m.cp_l = (T)m.cp_l;

@@ -1,0 +1,53 @@
+"""The register-resident operator kernels where their work split has edges: cell rows shorter and
+longer than a warp's group of cells, a last group that is partly empty, meshes of several rounds of
+the persistent grid (the cells are walked with carries), one cell, and Dirichlet faces that
+constrain some columns only; against the oracle, FP64 to 1e-12 and FP32 to 2e-5 (max norm)."""
+import numpy as np
+import pytest
+import torch
+
+from meltpooldg_b200 import heat as H
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+TOL64, TOL32 = 1e-12, 2e-5
+KT = dict(law=1, rho=1.0, cp=1.0, k=1.0, k1=0.5)
+# several rounds of the grid: more cells than 148 SMs x resident warps x cells per warp
+LONG = {1: (61, 47, 53), 2: (37, 41, 43), 3: (29, 31, 37), 4: (23, 29, 31)}
+
+
+def rel(a, b):
+    a = a.double().cpu().numpy()
+    return np.abs(a - b).max() / np.abs(b).max()
+
+
+@pytest.mark.parametrize("degree", [1, 2, 3, 4])
+@pytest.mark.parametrize("cells", [(1, 1, 1), (33, 1, 2), (2, 17, 3), "long"])
+@pytest.mark.parametrize("perturb", [0.0, 0.2])
+@pytest.mark.parametrize("mask", [0b111111, 0b010010])
+def test_operator_verbs(degree, cells, perturb, mask):
+    cells = LONG[degree] if cells == "long" else cells
+    if degree == 1 and min(cells) == 1 and mask == 0b111111:
+        mask = 0b000001  # otherwise every DoF is constrained
+    dt = 1e-3
+    o = O.Oracle(degree, cells, perturb=perturb, seed=5, dirichlet_mask=mask)
+    o.set_material(O.material(**KT), dt)
+    g = H.HeatDiffuseOperator(H.box_mesh(degree, cells, perturb=perturb, seed=5,
+                                         dirichlet=[f for f in range(6) if mask >> f & 1]))
+    g.set_material(H.material(**KT))
+    g.reset_time_increment(dt)
+    rng = np.random.default_rng(degree)
+    n = o.n_dofs
+    src, Tl, To, q = (rng.uniform(lo, 1.0, n) for lo in (-1.0, 0.0, 0.0, 0.0))
+    d = {k: torch.tensor(v, device="cuda") for k, v in dict(src=src, Tl=Tl, To=To, q=q).items()}
+    g.set_linearization(d["Tl"], d["To"])
+    ref = o.vmult(src, Tl, To)
+    assert rel(g.vmult(g.new_vector(), d["src"]), ref) <= TOL64
+    s32 = d["src"].float()
+    assert rel(g.vmult(g.new_vector(torch.float32), s32), ref) <= TOL32
+    assert rel(g.vmult_picard_f32(g.new_vector(torch.float32), s32),
+               o.vmult(src, Tl, To, form=2)) <= TOL32
+    assert rel(1.0 / g.inverse_diagonal_picard_f32(g.new_vector(torch.float32)),
+               1.0 / o.inverse_diagonal(Tl, To, form=2)) <= TOL32
+    assert rel(g.create_rhs(g.new_vector(), d["To"], d["q"]), o.create_rhs(Tl, To, q)) <= TOL64
