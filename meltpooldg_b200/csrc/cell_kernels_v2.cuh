@@ -653,9 +653,10 @@ __global__ void __launch_bounds__(32 * kV2Warps, (v2_min_blocks<n, T, GEO, LAW>(
 #pragma unroll
       for (int k = 0; k < n; ++k)
 #pragma unroll
-        for (int j = 0; j < n; ++j)
-          if (!cm.template at<n>(j, k))
-            dot += (double)__ldg(in + (rs * j + ps * k)) * (double)Q[k][j];
+        for (int j = 0; j < n; ++j) {
+          const T u = __ldg(in + (rs * j + ps * k));
+          dot += cm.template at<n>(j, k) ? 0.0 : (double)u * (double)Q[k][j];
+        }
     }
     bool mine = active;
     if constexpr (n == 3) {

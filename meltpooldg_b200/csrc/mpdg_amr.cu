@@ -13,8 +13,10 @@
 // same local indices and interpolates them in place with the 1D child matrices
 // I_s[j][a] = l_a((s + xi_j)/2), one direction at a time (lines along d on a hanging face
 // normal to another direction, or on a hanging edge parallel to d); the scatter applies the
-// transposes in the reverse order. One CTA of (p+1)^3 threads per cell, every sweep through
-// shared memory: the first GPU form of this path, written for parity.
+// transposes in the reverse order. The operator and the linearisation point's fields run on the
+// register-resident kernels of amr_cells.cuh; the residual and the diagonal, formed once per
+// Newton step and time step, with one CTA of (p+1)^3 threads per cell, every sweep through shared
+// memory.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -32,9 +34,12 @@
 #include <vector>
 
 #include "../../include/mpdg_heat.h"
+#include "amr_cells.cuh"
 #include "fe_tables.hpp"
 
 int mpdg_internal_fail(int code, const char *msg);
+
+using namespace mpdg;
 
 namespace {
 
@@ -44,15 +49,11 @@ constexpr int kLevelShift = 10;  // bits 10-12: the cell's refinement level
 constexpr int kAmrMaxLevel = 6;
 
 struct AmrArgs {
-  const int *idx;
+  const int *idx;  // [cell][i][k][j], Dirichlet DoFs complemented (amr_cells.cuh)
   const uint16_t *code;
-  const uint8_t *mask;
   const double *src;
   const double *Tl;
   const double *q;  // create_rhs: the nodal heat source (nullable)
-  // the linearisation point's values and reference gradients at the q-points, [cell][4][n^3],
-  // built once per solve (nullable: the operator evaluates T_lin itself)
-  const double *tf;
   double *dst;
   int64_t n_cells;
   double h[3];
@@ -71,6 +72,13 @@ int fail(int code, const std::string &msg) { return mpdg_internal_fail(code, msg
     const int rc_ = (call);        \
     if (rc_ != MPDG_OK) return rc_; \
   } while (0)
+
+// the index entry of node t (x fastest) of a cell
+template <int n> __device__ __forceinline__ int cell_entry(const AmrArgs &a, int64_t c, int t)
+{
+  const int i = t % n, j = (t / n) % n, k = t / (n * n);
+  return a.idx[c * (n * n * n) + i * n * n + k * n + j];
+}
 
 // out[t] = sum_a M[o][a] in[line(a)], o = t's index along dir (M row-major n x n);
 // transpose: sum_a M[a][o] in[line(a)]
@@ -195,71 +203,6 @@ __device__ __forceinline__ void apply_cell(const AmrArgs &a, double size, double
   integrate_cell<n>(a, u, val, gx, gy, gz, t1, t2, s1, s2, s3, t);
 }
 
-template <int n>
-__global__ void k_amr_vmult(const AmrArgs a)
-{
-  constexpr int n3 = n * n * n;
-  __shared__ double u[n3], T[n3], tmp[n3], t1[n3], t2[n3], s1[n3], s2[n3], s3[n3];
-  __shared__ double val[n3], gx[n3], gy[n3], gz[n3], Tv[n3], Tx[n3], Ty[n3], Tz[n3];
-  const int t = threadIdx.x;
-  for (int64_t c = blockIdx.x; c < a.n_cells; c += gridDim.x) {
-    const int code = a.code[c];
-    const int dof = a.idx[c * n3 + t];
-    const bool hang = (code & 0x1F8) != 0;
-    const double size = cell_size(code);
-    const bool eval_T = a.tangent && !a.tf;
-    u[t] = a.mask[dof] ? 0.0 : a.src[dof];
-    if (eval_T) T[t] = a.Tl[dof];
-    if (a.tangent && a.tf) {
-      const double *f = a.tf + c * 4 * n3;
-      Tv[t] = f[t];
-      Tx[t] = f[n3 + t];
-      Ty[t] = f[2 * n3 + t];
-      Tz[t] = f[3 * n3 + t];
-    }
-    __syncthreads();
-    if (hang) {
-      for (int d = 0; d < 3; ++d) {
-        const double *I = a.I[(code >> d) & 1];
-        hang_dir<n>(u, tmp, code, d, I, false, t);
-        if (eval_T) hang_dir<n>(T, tmp, code, d, I, false, t);
-      }
-    }
-    if (eval_T) evaluate<n>(a, T, Tv, Tx, Ty, Tz, t1, t2, s1, s2, s3, t);
-    apply_cell<n>(a, size, u, Tv, Tx, Ty, Tz, val, gx, gy, gz, t1, t2, s1, s2, s3, t);
-    if (hang) {
-      for (int d = 2; d >= 0; --d) hang_dir<n>(u, tmp, code, d, a.I[(code >> d) & 1], true, t);
-    }
-    if (!a.mask[dof]) atomicAdd(a.dst + dof, u[t]);
-    __syncthreads();
-  }
-}
-
-// the linearisation point's values and reference gradients at the q-points of every cell
-// (hanging interpolation applied), [cell][4][n^3]: the operator's T_lin evaluation, once per solve
-template <int n>
-__global__ void k_amr_tfields(const AmrArgs a, double *tf)
-{
-  constexpr int n3 = n * n * n;
-  __shared__ double T[n3], tmp[n3], t1[n3], t2[n3], s1[n3], s2[n3], s3[n3];
-  __shared__ double Tv[n3], Tx[n3], Ty[n3], Tz[n3];
-  const int t = threadIdx.x;
-  for (int64_t c = blockIdx.x; c < a.n_cells; c += gridDim.x) {
-    const int code = a.code[c];
-    T[t] = a.Tl[a.idx[c * n3 + t]];
-    __syncthreads();
-    if ((code & 0x1F8) != 0)
-      for (int d = 0; d < 3; ++d) hang_dir<n>(T, tmp, code, d, a.I[(code >> d) & 1], false, t);
-    evaluate<n>(a, T, Tv, Tx, Ty, Tz, t1, t2, s1, s2, s3, t);
-    double *f = tf + c * 4 * n3;
-    f[t] = Tv[t];
-    f[n3 + t] = Tx[t];
-    f[2 * n3 + t] = Ty[t];
-    f[3 * n3 + t] = Tz[t];
-    __syncthreads();
-  }
-}
-
 // diag(F^T A_e F) per cell at its gathered DoFs (distinct within a cell), by applying the
 // cell operator to the cell's unit vectors (a cell on a hanging interface has no closed form)
 template <int n>
@@ -271,7 +214,7 @@ __global__ void k_amr_diag(const AmrArgs a)
   const int t = threadIdx.x;
   for (int64_t c = blockIdx.x; c < a.n_cells; c += gridDim.x) {
     const int code = a.code[c];
-    const int dof = a.idx[c * n3 + t];
+    const int entry = cell_entry<n>(a, c, t), dof = amr_dof(entry);
     const bool hang = (code & 0x1F8) != 0;
     const double size = cell_size(code);
     if (a.tangent) {
@@ -332,7 +275,7 @@ __global__ void k_amr_diag(const AmrArgs a)
         __syncthreads();
       }
     }
-    if (!a.mask[dof]) atomicAdd(a.dst + dof, mine);
+    if (entry >= 0) atomicAdd(a.dst + dof, mine);
     __syncthreads();
   }
 }
@@ -348,7 +291,7 @@ __global__ void k_amr_rhs(const AmrArgs a)
   const int t = threadIdx.x;
   for (int64_t c = blockIdx.x; c < a.n_cells; c += gridDim.x) {
     const int code = a.code[c];
-    const int dof = a.idx[c * n3 + t];
+    const int entry = cell_entry<n>(a, c, t), dof = amr_dof(entry);
     const bool hang = (code & 0x1F8) != 0;
     const double size = cell_size(code);
     T[t] = a.Tl[dof];
@@ -384,13 +327,12 @@ __global__ void k_amr_rhs(const AmrArgs a)
     if (hang) {
       for (int d = 2; d >= 0; --d) hang_dir<n>(u, tmp, code, d, a.I[(code >> d) & 1], true, t);
     }
-    if (!a.mask[dof]) atomicAdd(a.dst + dof, u[t]);
+    if (entry >= 0) atomicAdd(a.dst + dof, u[t]);
     __syncthreads();
   }
 }
 
-// vector kernels of the Krylov solve on the refined mesh (sums by block reduction and one
-// atomic add per block into a device scalar)
+// a . b (block reduction and one atomic add per block into a device scalar)
 __global__ void k_amr_dot(int64_t n, const double *__restrict__ a, const double *__restrict__ b,
                           double *out)
 {
@@ -415,15 +357,6 @@ __global__ void k_amr_axpby(int64_t n, double a, const double *__restrict__ x, d
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x)
     y[i] = a * x[i] + b * y[i];
-}
-
-// z = D r
-__global__ void k_amr_mul(int64_t n, const double *__restrict__ D, const double *__restrict__ r,
-                          double *z)
-{
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x)
-    z[i] = D[i] * r[i];
 }
 
 // d <- |d| > 1e-10 ? 1/d : 1 (Dirichlet DoFs, left zero, become 1)
@@ -472,8 +405,11 @@ struct mpdg_amr {
   uint16_t *d_code = nullptr;
   uint8_t *d_mask = nullptr;
   // Krylov / step workspace (n_dofs each) and a device scalar for the sums
-  double *w[7] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+  double *w[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
   double *d_sum = nullptr;
+  AmrCg *cg = nullptr;         // the CG iteration's scalars
+  double *partials = nullptr;  // grid reductions: 2 x kAmrMaxBlocks partial sums
+  unsigned *counter = nullptr;
   double *tf = nullptr;  // tangent fields of the solve's linearisation point, [cell][4][n^3]
 };
 
@@ -503,6 +439,12 @@ void release(mpdg_amr *h)
   h->d_sum = nullptr;
   if (h->tf) cudaFree(h->tf);
   h->tf = nullptr;
+  if (h->cg) cudaFree(h->cg);
+  h->cg = nullptr;
+  if (h->partials) cudaFree(h->partials);
+  h->partials = nullptr;
+  if (h->counter) cudaFree(h->counter);
+  h->counter = nullptr;
 }
 
 // the host description: active cells, node numbering, hanging nodes, DoFs, cell data
@@ -724,6 +666,26 @@ int build_host(mpdg_amr *h, const mpdg_mesh_desc *desc, const uint8_t *refine)
 
 }  // namespace
 
+namespace {
+
+// the 1D tables of this translation unit's kernels, once per device
+cudaError_t upload_tables(int device)
+{
+  static std::mutex mu;
+  static bool done[64] = {};
+  if (device < 0 || device >= 64) return cudaErrorInvalidDevice;
+  std::lock_guard<std::mutex> lock(mu);
+  if (done[device]) return cudaSuccess;
+  std::vector<double> tab, w, xl;
+  fill_even_odd(tab, w, xl);
+  cudaError_t e = cudaMemcpyToSymbol(c_tab_d, tab.data(), sizeof(double) * kTabSize);
+  if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_w_d, w.data(), sizeof(double) * kWTabSize);
+  done[device] = e == cudaSuccess;
+  return e;
+}
+
+}  // namespace
+
 extern "C" int mpdg_amr_create(const mpdg_mesh_desc *desc, const uint8_t *refine, int device,
                                mpdg_amr **out)
 {
@@ -787,7 +749,26 @@ extern "C" int mpdg_amr_create(const mpdg_mesh_desc *desc, const uint8_t *refine
   }
   if (device >= 0) {
     const int n3 = h->n * h->n * h->n;
-    std::vector<int> idx32(h->cell_dofs.begin(), h->cell_dofs.end());
+    // device order: the cells with a hanging face or edge first, so that few warps interpolate and
+    // the longest ones start first; a cell's entries as [i][k][j], Dirichlet DoFs complemented
+    const int n = h->n;
+    std::vector<int> entry((size_t)h->n_dofs);
+    for (int64_t v = 0; v < h->n_dofs; ++v)
+      entry[(size_t)v] = h->mask[(size_t)v] ? ~(int)v : (int)v;
+    std::vector<int> idx32((size_t)h->n_cells * n3);
+    std::vector<uint16_t> codes((size_t)h->n_cells);
+    int64_t at = 0;
+    for (int hang = 1; hang >= 0; --hang)
+      for (int64_t c = 0; c < h->n_cells; ++c) {
+        if (((h->codes[(size_t)c] & 0x1F8) != 0) != (hang == 1)) continue;
+        const int64_t *from = &h->cell_dofs[(size_t)c * n3];
+        int *to = &idx32[(size_t)at * n3];
+        for (int k = 0; k < n; ++k)
+          for (int j = 0; j < n; ++j)
+            for (int i = 0; i < n; ++i)
+              to[i * n * n + k * n + j] = entry[(size_t)*from++];
+        codes[(size_t)at++] = h->codes[(size_t)c];
+      }
     cudaError_t e = cudaSetDevice(device);
     if (e == cudaSuccess) e = cudaMalloc(&h->d_idx, sizeof(int) * idx32.size());
     if (e == cudaSuccess) e = cudaMalloc(&h->d_code, sizeof(uint16_t) * h->codes.size());
@@ -795,11 +776,11 @@ extern "C" int mpdg_amr_create(const mpdg_mesh_desc *desc, const uint8_t *refine
     if (e == cudaSuccess)
       e = cudaMemcpy(h->d_idx, idx32.data(), sizeof(int) * idx32.size(), cudaMemcpyHostToDevice);
     if (e == cudaSuccess)
-      e = cudaMemcpy(h->d_code, h->codes.data(), sizeof(uint16_t) * h->codes.size(),
+      e = cudaMemcpy(h->d_code, codes.data(), sizeof(uint16_t) * codes.size(),
                      cudaMemcpyHostToDevice);
     if (e == cudaSuccess)
       e = cudaMemcpy(h->d_mask, h->mask.data(), h->mask.size(), cudaMemcpyHostToDevice);
-    (void)n3;
+    if (e == cudaSuccess) e = upload_tables(device);
     if (e != cudaSuccess) {
       release(h);
       delete h;
@@ -880,7 +861,6 @@ AmrArgs make_args(const mpdg_amr *h, const double *T_lin)
   std::memset(&a, 0, sizeof(a));
   a.idx = h->d_idx;
   a.code = h->d_code;
-  a.mask = h->d_mask;
   a.Tl = T_lin;
   a.n_cells = h->n_cells;
   for (int d = 0; d < 3; ++d) a.h[d] = h->h[d];
@@ -904,10 +884,11 @@ AmrArgs make_args(const mpdg_amr *h, const double *T_lin)
   return a;
 }
 
-enum { CELL_VMULT = 0, CELL_DIAG = 1, CELL_RHS = 2 };
+enum { CELL_DIAG = 1, CELL_RHS = 2 };
 
-// a persistent grid of as many CTAs (one cell each at a time) as the SMs hold at once
-template <typename K> int resident_grid(K kernel, int threads, int64_t n_cells)
+// a persistent grid of as many CTAs as the SMs hold at once, for n_jobs CTAs' worth of work
+constexpr int kAmrMaxBlocks = 148 * 32;
+template <typename K> int resident_grid(K kernel, int threads, int64_t n_jobs, size_t smem = 0)
 {
   static std::mutex mu;
   static std::map<const void *, int> per_sm_of;  // per kernel
@@ -922,24 +903,76 @@ template <typename K> int resident_grid(K kernel, int threads, int64_t n_cells)
     }
     auto it = per_sm_of.find(reinterpret_cast<const void *>(kernel));
     if (it == per_sm_of.end()) {
-      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0) != cudaSuccess ||
+      if (smem > 48 * 1024)
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) !=
+            cudaSuccess ||
           per_sm < 1)
-        per_sm = 16;
+        per_sm = smem ? 1 : 16;
       per_sm_of[reinterpret_cast<const void *>(kernel)] = per_sm;
     } else {
       per_sm = it->second;
     }
   }
-  return (int)std::min<int64_t>(n_cells, (int64_t)per_sm * sms);
+  return (int)std::max<int64_t>(
+    1, std::min<int64_t>(std::min<int64_t>(n_jobs, kAmrMaxBlocks), (int64_t)per_sm * sms));
+}
+
+// arguments of the register-resident kernels
+AmrCellArgs make_cell_args(const mpdg_amr *h, const double *T_lin)
+{
+  AmrCellArgs a;
+  std::memset(&a, 0, sizeof(a));
+  a.idx = h->d_idx;
+  a.code = h->d_code;
+  a.Tl = T_lin;
+  a.n_cells = h->n_cells;
+  a.detJ = h->h[0] * h->h[1] * h->h[2];
+  for (int d = 0; d < 3; ++d) a.Gd[d] = a.detJ / (h->h[d] * h->h[d]);
+  a.cval = h->mat.rho_l * h->mat.cp_l / h->dt;
+  a.k0 = h->mat.k_l;
+  a.k1 = h->mat.law == MPDG_LAW_LINEAR_K ? h->mat.k1 : 0.0;
+  const int n = h->n;
+  const Tables1D tb = make_tables(n);
+  for (int j = 0; j < n; ++j)
+    for (int i = 0; i < n; ++i) a.I[j * n + i] = lagrange(tb.xl, n, i, 0.5 * tb.xl[j]);
+  return a;
+}
+
+template <int n, bool TANGENT, bool EVAL>
+void launch_apply(const AmrCellArgs &a, AmrCg *cg, double *partials, unsigned *counter)
+{
+  auto k = k_amr_apply<n, TANGENT, EVAL>;
+  constexpr size_t smem = amr_smem<n, EVAL>();
+  constexpr int cells = kV2Warps * v2_cells_per_warp<n>();
+  const int g = resident_grid(k, 32 * kV2Warps, (a.n_cells + cells - 1) / cells, smem);
+  k<<<g, 32 * kV2Warps, smem>>>(a, cg, partials, counter);
+}
+template <int n> void launch_tfields(const AmrCellArgs &a, double *tf)
+{
+  auto k = k_amr_tfields<n>;
+  constexpr size_t smem = amr_smem<n, false>();
+  constexpr int cells = kV2Warps * v2_cells_per_warp<n>();
+  const int g = resident_grid(k, 32 * kV2Warps, (a.n_cells + cells - 1) / cells, smem);
+  k<<<g, 32 * kV2Warps, smem>>>(a, tf);
+}
+template <int n>
+void launch_apply_n(const AmrCellArgs &a, bool tangent, AmrCg *cg, double *partials,
+                    unsigned *counter)
+{
+  if (!tangent)
+    launch_apply<n, false, false>(a, cg, partials, counter);
+  else if (a.tf)
+    launch_apply<n, true, false>(a, cg, partials, counter);
+  else
+    launch_apply<n, true, true>(a, cg, partials, counter);
 }
 
 template <int n>
 void launch_n(int kind, const AmrArgs &a)
 {
   constexpr int n3 = n * n * n;
-  if (kind == CELL_VMULT) {
-    k_amr_vmult<n><<<resident_grid(k_amr_vmult<n>, n3, a.n_cells), n3>>>(a);
-  } else if (kind == CELL_DIAG) {
+  if (kind == CELL_DIAG) {
     k_amr_diag<n><<<resident_grid(k_amr_diag<n>, n3, a.n_cells), n3>>>(a);
   } else {
     k_amr_rhs<n><<<resident_grid(k_amr_rhs<n>, n3, a.n_cells), n3>>>(a);
@@ -975,6 +1008,12 @@ int sync_status()
 
 int vgrid(int64_t n) { return (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 148 * 8)); }
 
+// a reduction over n values: two blocks of 512 threads per SM (fewer partial sums for the last one)
+int reduce_grid(int64_t n)
+{
+  return (int)std::max<int64_t>(1, std::min<int64_t>((n + 511) / 512, 148 * 2));
+}
+
 // the tangent fields of T_lin into h->tf (for the applications of one solve)
 int tfields_impl(mpdg_amr *h, const double *T_lin)
 {
@@ -986,29 +1025,42 @@ int tfields_impl(mpdg_amr *h, const double *T_lin)
       return fail(MPDG_ERR_OUT_OF_MEMORY, std::string("cudaMalloc: ") + cudaGetErrorString(e));
     }
   }
-  AmrArgs a = make_args(h, T_lin);
-  const int64_t nc = h->n_cells;
+  const AmrCellArgs a = make_cell_args(h, T_lin);
   switch (h->n) {
-    case 2: k_amr_tfields<2><<<resident_grid(k_amr_tfields<2>, 8, nc), 8>>>(a, h->tf); break;
-    case 3: k_amr_tfields<3><<<resident_grid(k_amr_tfields<3>, 27, nc), 27>>>(a, h->tf); break;
-    case 4: k_amr_tfields<4><<<resident_grid(k_amr_tfields<4>, 64, nc), 64>>>(a, h->tf); break;
-    case 5: k_amr_tfields<5><<<resident_grid(k_amr_tfields<5>, 125, nc), 125>>>(a, h->tf); break;
+    case 2: launch_tfields<2>(a, h->tf); break;
+    case 3: launch_tfields<3>(a, h->tf); break;
+    case 4: launch_tfields<4>(a, h->tf); break;
+    case 5: launch_tfields<5>(a, h->tf); break;
     default: return fail(MPDG_ERR_INVALID_ARGUMENT, "degree");
   }
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? MPDG_OK : fail(MPDG_ERR_CUDA, cudaGetErrorString(e));
 }
 
-int vmult_impl(mpdg_amr *h, double *dst, const double *src, const double *T_lin,
-               const double *tf = nullptr)
+bool is_tangent(const mpdg_amr *h) { return h->mat.law == MPDG_LAW_LINEAR_K && h->mat.k1 != 0.0; }
+
+// a.dst += J a.src; with cg the sum src.dst, which sets its alpha
+int apply_cells(const mpdg_amr *h, const AmrCellArgs &a, AmrCg *cg = nullptr)
 {
-  AmrArgs a = make_args(h, T_lin);
+  const bool tangent = is_tangent(h);
+  switch (h->n) {
+    case 2: launch_apply_n<2>(a, tangent, cg, h->partials, h->counter); break;
+    case 3: launch_apply_n<3>(a, tangent, cg, h->partials, h->counter); break;
+    case 4: launch_apply_n<4>(a, tangent, cg, h->partials, h->counter); break;
+    case 5: launch_apply_n<5>(a, tangent, cg, h->partials, h->counter); break;
+    default: return fail(MPDG_ERR_INVALID_ARGUMENT, "degree");
+  }
+  const cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? MPDG_OK : fail(MPDG_ERR_CUDA, cudaGetErrorString(e));
+}
+
+int vmult_impl(mpdg_amr *h, double *dst, const double *src, const double *T_lin)
+{
+  AmrCellArgs a = make_cell_args(h, T_lin);
   a.src = src;
   a.dst = dst;
-  a.tf = a.tangent ? tf : nullptr;
-  if (!a.tangent) a.Tl = src;
   k_amr_zero<<<vgrid(h->n_dofs), 256>>>(h->n_dofs, dst);
-  return launch_cells(h, CELL_VMULT, a);
+  return apply_cells(h, a);
 }
 
 int diag_impl(mpdg_amr *h, double *inv, const double *T_lin)
@@ -1042,13 +1094,19 @@ int ensure_workspace(mpdg_amr *h)
         return fail(MPDG_ERR_OUT_OF_MEMORY, std::string("cudaMalloc: ") + cudaGetErrorString(e));
       }
     }
-  if (!h->d_sum) {
-    const cudaError_t e = cudaMalloc(&h->d_sum, sizeof(double));
-    if (e != cudaSuccess) {
-      h->d_sum = nullptr;
-      return fail(MPDG_ERR_OUT_OF_MEMORY, std::string("cudaMalloc: ") + cudaGetErrorString(e));
-    }
-  }
+  auto get = [](auto *&p, size_t bytes) -> int {
+    if (p) return MPDG_OK;
+    cudaError_t e = cudaMalloc(&p, bytes);
+    if (e == cudaSuccess) e = cudaMemset(p, 0, bytes);
+    if (e == cudaSuccess) return MPDG_OK;
+    if (p) cudaFree(p);
+    p = nullptr;
+    return fail(MPDG_ERR_OUT_OF_MEMORY, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+  };
+  TRY_AMR(get(h->d_sum, sizeof(double)));
+  TRY_AMR(get(h->cg, sizeof(AmrCg)));
+  TRY_AMR(get(h->partials, sizeof(double) * 2 * kAmrMaxBlocks));
+  TRY_AMR(get(h->counter, sizeof(unsigned)));
   return MPDG_OK;
 }
 
@@ -1060,48 +1118,49 @@ int dot(mpdg_amr *h, const double *a, const double *b, double *out)
   return e == cudaSuccess ? MPDG_OK : fail(MPDG_ERR_CUDA, cudaGetErrorString(e));
 }
 
-// Jacobi-CG (deal.II SolverCG semantics, ReductionControl) on the refined mesh: x from 0
+// Jacobi-CG (deal.II SolverCG semantics, ReductionControl) on the refined mesh: x from 0. The
+// scalars stay on the device and every kernel returns at once after convergence, so an iteration
+// is three launches and the host reads the state once per kAmrChunk of them; with a host read per
+// sum and one kernel per vector operation it was eight launches and three synchronisations.
+constexpr int kAmrChunk = 8;
 int cg_impl(mpdg_amr *h, double *x, const double *b, const double *inv, const double *T_lin,
             double rel_tol, double abs_tol, int max_it, int *iterations)
 {
   TRY_AMR(ensure_workspace(h));
   const int64_t N = h->n_dofs;
-  const int g = vgrid(N);
-  double *r = h->w[0], *z = h->w[1], *p = h->w[2], *Ap = h->w[3];
-  k_amr_zero<<<g, 256>>>(N, x);
-  k_amr_axpby<<<g, 256>>>(N, 1.0, b, 0.0, r);
-  k_amr_mul<<<g, 256>>>(N, inv, r, z);
-  k_amr_axpby<<<g, 256>>>(N, 1.0, z, 0.0, p);
-  double rr = 0.0, rz = 0.0;
-  TRY_AMR(dot(h, r, r, &rr));
-  TRY_AMR(dot(h, r, z, &rz));
-  const double tol = std::max(abs_tol, rel_tol * std::sqrt(rr));
+  const int g = vgrid(N), gr = reduce_grid(N);
+  double *r = h->w[0], *p = h->w[1], *Ap = h->w[2];
   *iterations = 0;
-  if (std::sqrt(rr) <= tol) return MPDG_OK;
-  // T_lin is fixed during the solve: its values and gradients at the q-points once
-  const double *tf = nullptr;
-  if (T_lin && h->mat.law == MPDG_LAW_LINEAR_K && h->mat.k1 != 0.0) {
+  k_amr_cg_init<<<g, 256>>>(N, b, inv, x, r, p, Ap, h->cg, h->partials, h->counter, rel_tol,
+                            abs_tol, max_it);
+  AmrCellArgs a = make_cell_args(h, T_lin);
+  a.src = p;
+  a.dst = Ap;
+  if (T_lin && is_tangent(h)) {  // T_lin is fixed during the solve: its fields once
     TRY_AMR(tfields_impl(h, T_lin));
-    tf = h->tf;
+    a.tf = h->tf;
   }
-  for (int it = 1; it <= max_it; ++it) {
-    TRY_AMR(vmult_impl(h, Ap, p, T_lin, tf));
-    double pap = 0.0;
-    TRY_AMR(dot(h, p, Ap, &pap));
-    if (!(pap > 0.0)) return fail(MPDG_ERR_BREAKDOWN, "CG breakdown: p.Ap <= 0");
-    const double alpha = rz / pap;
-    k_amr_axpby<<<g, 256>>>(N, alpha, p, 1.0, x);
-    k_amr_axpby<<<g, 256>>>(N, -alpha, Ap, 1.0, r);
-    TRY_AMR(dot(h, r, r, &rr));
-    if (!std::isfinite(rr)) return fail(MPDG_ERR_NAN, "CG residual is not finite");
-    *iterations = it;
-    if (std::sqrt(rr) <= tol) return MPDG_OK;
-    k_amr_mul<<<g, 256>>>(N, inv, r, z);
-    double rz_new = 0.0;
-    TRY_AMR(dot(h, r, z, &rz_new));
-    k_amr_axpby<<<g, 256>>>(N, 1.0, z, rz_new / rz, p);
-    rz = rz_new;
+  AmrCg st;
+  for (;;) {
+    for (int i = 0; i < kAmrChunk; ++i) {
+      TRY_AMR(apply_cells(h, a, h->cg));
+      k_amr_cg_update<<<gr, 512>>>(N, inv, Ap, r, h->cg, h->partials, h->counter);
+      k_amr_cg_direction<<<g, 256>>>(N, inv, r, x, p, Ap, h->cg);
+    }
+    const cudaError_t e = cudaMemcpy(&st, h->cg, sizeof(st), cudaMemcpyDeviceToHost);
+    if (e != cudaSuccess) return fail(MPDG_ERR_CUDA, cudaGetErrorString(e));
+    if (st.done) break;
   }
+  // the last iteration's step (none was taken by a solve that ended before or at a breakdown)
+  if (st.it > 0 && st.status != MPDG_ERR_BREAKDOWN) {
+    k_amr_cg_last<<<g, 256>>>(N, p, x, h->cg);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return fail(MPDG_ERR_CUDA, cudaGetErrorString(e));
+  }
+  *iterations = st.status == MPDG_ERR_NAN ? st.it - 1 : st.it;
+  if (st.done == 1) return MPDG_OK;
+  if (st.status == MPDG_ERR_BREAKDOWN) return fail(MPDG_ERR_BREAKDOWN, "CG breakdown: p.Ap <= 0");
+  if (st.status == MPDG_ERR_NAN) return fail(MPDG_ERR_NAN, "CG residual is not finite");
   return fail(MPDG_ERR_NOT_CONVERGED, "CG on the hanging-node mesh did not converge");
 }
 
@@ -1111,8 +1170,7 @@ extern "C" int mpdg_amr_vmult(mpdg_amr *h, double *dst, const double *src, const
 {
   if (!h || !dst || !src) return fail(MPDG_ERR_INVALID_ARGUMENT, "null argument");
   TRY_AMR(ready(h));
-  const bool tangent = h->mat.law == MPDG_LAW_LINEAR_K && h->mat.k1 != 0.0;
-  if (tangent && !T_lin)
+  if (is_tangent(h) && !T_lin)
     return fail(MPDG_ERR_INVALID_ARGUMENT, "LINEAR_K needs the linearisation point");
   TRY_AMR(check_device_vectors({dst, src, T_lin}));
   TRY_AMR(vmult_impl(h, dst, src, T_lin));
@@ -1123,8 +1181,7 @@ extern "C" int mpdg_amr_inverse_diagonal(mpdg_amr *h, double *inv_diag, const do
 {
   if (!h || !inv_diag) return fail(MPDG_ERR_INVALID_ARGUMENT, "null argument");
   TRY_AMR(ready(h));
-  const bool tangent = h->mat.law == MPDG_LAW_LINEAR_K && h->mat.k1 != 0.0;
-  if (tangent && !T_lin)
+  if (is_tangent(h) && !T_lin)
     return fail(MPDG_ERR_INVALID_ARGUMENT, "LINEAR_K needs the linearisation point");
   TRY_AMR(check_device_vectors({inv_diag, T_lin}));
   TRY_AMR(diag_impl(h, inv_diag, T_lin));
@@ -1147,13 +1204,12 @@ extern "C" int mpdg_amr_linear_solve(mpdg_amr *h, double *x, const double *b, co
 {
   if (!h || !x || !b) return fail(MPDG_ERR_INVALID_ARGUMENT, "null argument");
   TRY_AMR(ready(h));
-  const bool tangent = h->mat.law == MPDG_LAW_LINEAR_K && h->mat.k1 != 0.0;
-  if (tangent && !T_lin)
+  if (is_tangent(h) && !T_lin)
     return fail(MPDG_ERR_INVALID_ARGUMENT, "LINEAR_K needs the linearisation point");
   TRY_AMR(check_device_vectors({x, b, T_lin}));
   TRY_AMR(ensure_workspace(h));
   int its = 0;
-  double *inv = h->w[4];
+  double *inv = h->w[3];
   TRY_AMR(diag_impl(h, inv, T_lin));
   const int rc = cg_impl(h, x, b, inv, T_lin, rel_tolerance, abs_tolerance, max_iterations, &its);
   if (iterations) *iterations = its;
@@ -1181,7 +1237,7 @@ extern "C" int mpdg_amr_time_step(mpdg_amr *h, double dt, double dt_old, double 
                      ? dt / dt_old : 0.0;
   k_amr_predict<<<g, 256>>>(N, r, T_cur, T_old, h->d_mask);
   const bool tangent = h->mat.law == MPDG_LAW_LINEAR_K && h->mat.k1 != 0.0;
-  double *rhs = h->w[5], *delta = h->w[6], *inv = h->w[4];
+  double *rhs = h->w[4], *delta = h->w[5], *inv = h->w[3];
   TRY_AMR(diag_impl(h, inv, tangent ? T_cur : nullptr));
   // Newton-Raphson (newton_raphson_solver.cpp:22-68): rhs = -R(T); J delta = rhs; converged
   // when |rhs| < tol_res and |delta| < tol_corr (the converged update is not applied)

@@ -172,3 +172,37 @@ def test_implicit_steps_on_refined_mesh_match_oracle(mesh):
         dt_old = dt
         assert _relmax(Tg, T) <= 1e-9, step
         assert _relmax(Tog, To) <= 1e-9, step
+
+
+@pytest.mark.parametrize("p,cells", [(1, (61, 47, 53)), (2, (41, 37, 29)), (3, (31, 29, 23)),
+                                     (4, (23, 21, 25))])
+def test_many_cells_match_structured_operator(p, cells):
+    """More cells than one round of the operator kernel's grid holds, the last group of a warp
+    partly empty; the k(T) tangent evaluated in the kernel and from the solve's fields."""
+    mesh = H.box_mesh(p, cells, **BOX)
+    amr, st = AmrHeatOperator(mesh, (), device=0), H.HeatDiffuseOperator(mesh)
+    m = H.material(law=L.LAW_LINEAR_K, k=1.0, k1=0.5)
+    amr.set_material(m, 5e-3)
+    st.set_material(m)
+    st.reset_time_increment(5e-3)
+    g = torch.Generator(device="cuda").manual_seed(p)
+    T, x = (torch.rand(st.n_dofs, dtype=torch.float64, device="cuda", generator=g)
+            for _ in range(2))
+    st.set_linearization(T, T)
+    y, ref = torch.empty_like(x), st.vmult(st.new_vector(), x)
+    amr.vmult(y, x, T)
+    assert (y - ref).abs().max().item() <= 1e-12 * ref.abs().max().item()
+    its = amr.linear_solve(y, ref, T, rel_tolerance=1e-12)  # over free DoFs: y = x there
+    free = torch.tensor(amr.constraint_mask() == 0, device="cuda")
+    assert its > 8 and ((y - x) * free).abs().max().item() <= 1e-8
+
+
+def test_solve_stops_at_the_iteration_limit():
+    op = AmrHeatOperator(H.box_mesh(2, (4, 3, 3), **BOX), REFINE, device=0)
+    op.set_material(H.material(), 1e-2)
+    b = torch.ones(op.n_dofs, dtype=torch.float64, device="cuda")
+    b[torch.tensor(op.constraint_mask() != 0, device="cuda")] = 0.0
+    for limit in (0, 1, 9):  # none, one and more than one batch of launched iterations
+        with pytest.raises(H.ExcNoConvergence):
+            op.linear_solve(torch.empty_like(b), b, None, rel_tolerance=1e-15,
+                            max_iterations=limit)
