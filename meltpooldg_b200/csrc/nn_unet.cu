@@ -20,10 +20,10 @@
 // output gradient, rounded to BF16, convolved with the flipped, channel-
 // transposed weights (packed beside the forward ones), FP32 out
 // (MPDG_UNET_TC_BWD=0 keeps them on the CUDA cores in FP32). The weight
-// gradients and the CUDA-core forward (MPDG_UNET_TC=0) use k_conv3d: a CTA
-// holds an 8x8x4 output tile and 16 output channels, stages one input
-// channel's tile plus halo and its 16 x 27 weights in shared memory at a time
-// and accumulates in FP32 registers.
+// gradients run on the CUDA cores in FP32 (nn_wgrad.cuh). The CUDA-core forward
+// (MPDG_UNET_TC=0) is k_conv3d: a CTA holds an 8x8x4 output tile and 16 output
+// channels, stages one input channel's tile plus halo and its 16 x 27 weights in
+// shared memory at a time and accumulates in FP32 registers.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -36,6 +36,7 @@
 
 #include "../../include/mpdg_heat.h"
 #include "nn_conv_tc.cuh"
+#include "nn_wgrad.cuh"
 #include "reduce.cuh"
 
 using namespace mpdg;
@@ -166,68 +167,6 @@ __global__ void __launch_bounds__(TP) k_conv3d(Grid3 g, int Ci, int Co, const TI
     if (MASK) r = __bfloat162float(mask[aidx(co, p, np)]) > 0.f ? r : 0.f;
     out[tidx<TO>(co, p, np)] = fromf<TO>(r);
   }
-}
-
-// dw[co][ci][o] += sum_p gout[co][p] in[ci][p + o - 1] ; db[co] += sum_p gout[co][p]
-// CTA: one 8x8x4 tile, 16 co x 16 ci, thread (co, ci) keeps 27 accumulators.
-constexpr int CIB = 8;  // 16 co x 8 ci per CTA keeps the staged tiles under 48 KB
-__global__ void __launch_bounds__(COB * CIB) k_conv3d_wgrad(Grid3 g, int Ci, int Co,
-                                                      const __nv_bfloat16 *__restrict__ in,
-                                                      const float *__restrict__ gout, float *dw,
-                                                      float *db)
-{
-  __shared__ float s_g[COB * TP];
-  __shared__ float s_in[CIB * HP];
-  const int tiles_x = (g.nx + TX - 1) / TX, tiles_y = (g.ny + TY - 1) / TY;
-  const int tile = blockIdx.x;
-  const int bx = (tile % tiles_x) * TX, by = ((tile / tiles_x) % tiles_y) * TY,
-            bz = (tile / (tiles_x * tiles_y)) * TZ;
-  const int co0 = blockIdx.y * COB, ci0 = blockIdx.z * CIB;
-  const int64_t np = g.n();
-  for (int i = threadIdx.x; i < COB * TP; i += blockDim.x) {
-    const int c = i / TP, t = i % TP;
-    const int x = bx + t % TX, y = by + (t / TX) % TY, z = bz + t / (TX * TY);
-    const int co = co0 + c;
-    float v = 0.f;
-    if (co < Co && x < g.nx && y < g.ny && z < g.nz)
-      v = gout[(int64_t)co * np + x + (int64_t)g.nx * (y + (int64_t)g.ny * z)];
-    s_g[i] = v;
-  }
-  for (int i = threadIdx.x; i < CIB * HP; i += blockDim.x) {
-    const int c = i / HP, hh = i % HP;
-    const int hx = hh % HX, hy = (hh / HX) % HY, hz = hh / (HX * HY);
-    const int gx = bx + hx - 1, gy = by + hy - 1, gz = bz + hz - 1;
-    const int ci = ci0 + c;
-    float v = 0.f;
-    if (ci < Ci && gx >= 0 && gx < g.nx && gy >= 0 && gy < g.ny && gz >= 0 && gz < g.nz)
-      v = __bfloat162float(in[aidx(ci, gx + (int64_t)g.nx * (gy + (int64_t)g.ny * gz), np)]);
-    s_in[i] = v;
-  }
-  __syncthreads();
-  const int c = threadIdx.x / CIB, k = threadIdx.x % CIB;  // c: co offset, k: ci offset
-  float acc[27];
-#pragma unroll
-  for (int o = 0; o < 27; ++o) acc[o] = 0.f;
-  float bsum = 0.f;
-  for (int t = 0; t < TP; ++t) {
-    const float gv = s_g[c * TP + t];
-    bsum += gv;
-    const int tx = t % TX, ty = (t / TX) % TY, tz = t / (TX * TY);
-    const float *sp = s_in + k * HP + tx + HX * (ty + HY * tz);
-#pragma unroll
-    for (int dz = 0; dz < 3; ++dz)
-#pragma unroll
-      for (int dy = 0; dy < 3; ++dy)
-#pragma unroll
-        for (int dx = 0; dx < 3; ++dx)
-          acc[dx + 3 * (dy + 3 * dz)] = fmaf(gv, sp[dx + HX * (dy + HY * dz)], acc[dx + 3 * (dy + 3 * dz)]);
-  }
-  const int co = co0 + c, ci = ci0 + k;
-  if (co < Co && ci < Ci) {
-#pragma unroll
-    for (int o = 0; o < 27; ++o) atomicAdd(dw + ((int64_t)co * Ci + ci) * 27 + o, acc[o]);
-  }
-  if (db && blockIdx.z == 0 && k == 0 && co < Co) atomicAdd(db + co, bsum);
 }
 
 __host__ __device__ inline Grid3 coarse(Grid3 g) { return {(g.nx + 1) / 2, (g.ny + 1) / 2, (g.nz + 1) / 2}; }
@@ -393,8 +332,6 @@ struct mpdg_unet {
   float *zero_bias = nullptr;    // 64 zeros
   bool wpk_dirty = true;      // pb changed since the last packing
   bool use_tc = true;         // forward convolutions on the tensor cores
-  bool training = false;      // forward keeps what the backward pass reads
-  bool ups_valid = false;     // u2, u1, u0 hold the upsampled decoder inputs
   // raised by a tensor-core convolution whose wait expired: page-locked mapped host memory
   // (tc_err is its device address), read by the host without a synchronisation
   int *tc_err = nullptr, *tc_err_host = nullptr;
@@ -437,15 +374,52 @@ int conv(mpdg_unet *u, Grid3 g, int Ci, int Co, const TI *in, const __nv_bfloat1
   return MPDG_OK;
 }
 
-int wgrad(mpdg_unet *u, Grid3 g, int l, const __nv_bfloat16 *in, const float *gout)
+template <int CI, int CG>
+int wgrad_t(mpdg_unet *u, const nn_wg::Args &args)
 {
-  const ConvL &L = u->L[l];
-  const int tiles = ((g.nx + TX - 1) / TX) * ((g.ny + TY - 1) / TY) * ((g.nz + TZ - 1) / TZ);
-  dim3 grid(tiles, (L.co + COB - 1) / COB, (L.ci + CIB - 1) / CIB);
-  k_conv3d_wgrad<<<grid, COB * CIB, 0, u->stream>>>(g, L.ci, L.co, in, gout, u->grad + L.woff,
-                                              u->grad + L.boff);
+  auto k = nn_wg::k_wgrad<CI, CG>;
+  nn_wg::Args a = args;
+  constexpr size_t smem = nn_wg::smem_bytes<CI, CG>();
+  NNCU(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  a.ci_groups = (a.ci + CI - 1) / CI;
+  const int blocks = a.ci_groups * ((a.co + 4 * CG - 1) / (4 * CG));
+  const int64_t tiles = (int64_t)((a.nx + nn_wg::kX - 1) / nn_wg::kX) *
+                        ((a.ny + nn_wg::kY - 1) / nn_wg::kY) *
+                        ((a.nz + nn_wg::kZ - 1) / nn_wg::kZ);
+  // three CTAs per SM over all channel blocks
+  const int gx = (int)std::max<int64_t>(
+    1, std::min<int64_t>(tiles, (3 * u->sm_count + blocks - 1) / blocks));
+  k<<<dim3(gx, blocks), nn_wg::kThreads, smem, u->stream>>>(a);
   NNCU(cudaGetLastError());
   return MPDG_OK;
+}
+
+// the weight and bias gradients of layer l; up_from: the input is that coarser grid's,
+// nearest-neighbour upsampled
+int wgrad(mpdg_unet *u, Grid3 g, int l, const __nv_bfloat16 *in, const float *gout,
+          const Grid3 *up_from = nullptr)
+{
+  const ConvL &L = u->L[l];
+  nn_wg::Args a;
+  std::memset(&a, 0, sizeof(a));
+  a.nx = g.nx;
+  a.ny = g.ny;
+  a.nz = g.nz;
+  a.ci = L.ci;
+  a.co = L.co;
+  a.up = up_from != nullptr;
+  a.sx = up_from ? up_from->nx : g.nx;
+  a.sy = up_from ? up_from->ny : g.ny;
+  a.sz = up_from ? up_from->nz : g.nz;
+  a.in = in;
+  a.g = gout;
+  a.dw = u->grad + L.woff;
+  a.db = u->grad + L.boff;
+  // the output layer (1 channel) and the input layer (3 channels) fill the block's rows with
+  // row groups instead of channels
+  if (L.ci <= 4) return wgrad_t<4, 4>(u, a);
+  if (L.co <= 4) return wgrad_t<16, 1>(u, a);
+  return wgrad_t<16, 4>(u, a);
 }
 
 const __nv_bfloat16 *W(mpdg_unet *u, int l) { return u->pb + u->L[l].woff; }
@@ -628,16 +602,12 @@ int forward(mpdg_unet *u)
   NNTRY(conv_relu(u, E3A, g[3], u->p2, u->a3));
   NNTRY(conv_relu(u, E3B, g[3], u->a3, u->e3));
   // decoder: with the tensor-core path the upsampling is fused into the halo load of
-  // the next convolution (the upsampled tensors are then formed only for training)
-  u->ups_valid = !u->use_tc || u->training;
+  // the next convolution (the backward pass reads the coarse tensors as well)
   if (u->use_tc) {
-    if (u->training) NNTRY(up(g[2], 64, u->e3, u->u2));
     NNTRY((conv_tc<true, true>(u, D2A, g[2], u->e3, u->e2, u->s2, &g[3])));
     NNTRY(conv_relu(u, D2B, g[2], u->s2, u->d2));
-    if (u->training) NNTRY(up(g[1], 48, u->d2, u->u1));
     NNTRY((conv_tc<true, true>(u, D1A, g[1], u->d2, u->e1, u->s1, &g[2])));
     NNTRY(conv_relu(u, D1B, g[1], u->s1, u->d1));
-    if (u->training) NNTRY(up(g[0], 32, u->d1, u->u0));
     NNTRY((conv_tc<true, true>(u, D0A, g[0], u->d1, u->e0, u->s0, &g[1])));
     NNTRY(conv_relu(u, D0B, g[0], u->s0, u->d0));
     return conv_tc<false, false>(u, OUT, g[0], u->d0, (const __nv_bfloat16 *)nullptr, u->y);
@@ -658,13 +628,6 @@ int forward(mpdg_unet *u)
 int backward(mpdg_unet *u, const float *gy)
 {
   const Grid3 *g = u->g;
-  if (!u->ups_valid) {  // an inference forward fused the upsampling: form its outputs now
-    k_up<<<grid1d(g[2].n() * 64), 256, 0, u->stream>>>(g[2], 64, u->e3, u->u2);
-    k_up<<<grid1d(g[1].n() * 48), 256, 0, u->stream>>>(g[1], 48, u->d2, u->u1);
-    k_up<<<grid1d(g[0].n() * 32), 256, 0, u->stream>>>(g[0], 32, u->d1, u->u0);
-    NNCU(cudaGetLastError());
-    u->ups_valid = true;
-  }
   NNCU(cudaMemsetAsync(u->grad, 0, sizeof(float) * u->n_params, u->stream));
   float *gA = u->gA, *gB = u->gB, *gC = u->gC;
   auto relu_mask = [&](Grid3 gr, int C, const __nv_bfloat16 *y, float *gg) -> int {
@@ -692,21 +655,21 @@ int backward(mpdg_unet *u, const float *gy)
   NNTRY(dgrad(u, OUT, g[0], gy, gA, u->d0));            // gA: pre-relu of d0
   NNTRY(wgrad(u, g[0], D0B, u->s0, gA));
   NNTRY(dgrad(u, D0B, g[0], gA, gB, u->s0));            // gB: pre-relu of s0
-  NNTRY(wgrad(u, g[0], D0A, u->u0, gB));
+  NNTRY(wgrad(u, g[0], D0A, u->d1, gB, &g[1]));
   NNCU(cudaMemcpyAsync(u->gE0, gB, sizeof(float) * 16 * g[0].n(), cudaMemcpyDeviceToDevice, u->stream));
   NNTRY(dgrad(u, D0A, g[0], gB, gC, nullptr));          // gC: d u0 (32 @ g0)
   NNTRY(up_bwd(g[0], 32, gC, gA));                      // gA: d d1 (32 @ g1)
   NNTRY(relu_mask(g[1], 32, u->d1, gA));
   NNTRY(wgrad(u, g[1], D1B, u->s1, gA));
   NNTRY(dgrad(u, D1B, g[1], gA, gB, u->s1));
-  NNTRY(wgrad(u, g[1], D1A, u->u1, gB));
+  NNTRY(wgrad(u, g[1], D1A, u->d2, gB, &g[2]));
   NNCU(cudaMemcpyAsync(u->gE1, gB, sizeof(float) * 32 * g[1].n(), cudaMemcpyDeviceToDevice, u->stream));
   NNTRY(dgrad(u, D1A, g[1], gB, gC, nullptr));          // d u1 (48 @ g1)
   NNTRY(up_bwd(g[1], 48, gC, gA));                      // d d2 (48 @ g2)
   NNTRY(relu_mask(g[2], 48, u->d2, gA));
   NNTRY(wgrad(u, g[2], D2B, u->s2, gA));
   NNTRY(dgrad(u, D2B, g[2], gA, gB, u->s2));
-  NNTRY(wgrad(u, g[2], D2A, u->u2, gB));
+  NNTRY(wgrad(u, g[2], D2A, u->e3, gB, &g[3]));
   NNCU(cudaMemcpyAsync(u->gE2, gB, sizeof(float) * 48 * g[2].n(), cudaMemcpyDeviceToDevice, u->stream));
   NNTRY(dgrad(u, D2A, g[2], gB, gC, nullptr));          // d u2 (64 @ g2)
   NNTRY(up_bwd(g[2], 64, gC, gA));                      // d e3 (64 @ g3)
@@ -927,9 +890,7 @@ extern "C" int mpdg_unet_train_step(mpdg_unet *u, const float *input, const floa
 {
   if (!u || !input || !target) return nn_fail(MPDG_ERR_INVALID_ARGUMENT, "null argument");
   const int64_t n0 = u->g[0].n();
-  u->training = true;
   const int frc = mpdg_unet_forward(u, input, nullptr);
-  u->training = false;
   NNTRY(frc);
   float *gy = u->gC;  // reuse scratch for dL/dy (copied before backward overwrites gC)
   k_mse<<<grid1d(n0), 256, 0, u->stream>>>(n0, u->y, target, gy, u->partials, u->counter, u->lossd);

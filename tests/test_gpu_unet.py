@@ -152,3 +152,38 @@ def test_tensor_core_backward_matches_cuda_core_backward(monkeypatch):
     cos = torch.dot(a, b) / (a.norm() * b.norm())
     assert cos > 0.9999, cos
     assert (a - b).norm() / b.norm() < 2e-2
+
+
+@pytest.mark.parametrize("dims", [(8, 8, 8), (15, 8, 12), (16, 9, 13), (31, 17, 10), (47, 21, 33)])
+def test_weight_gradients_at_tile_edges_are_exact(dims):
+    """Weight and bias gradients of the last two layers (16 -> 1 and 16 -> 16) where every sum is
+    exact in FP32: constant inputs (biases, powers of two), an output layer with only its centre
+    tap, integer output gradients. Grids smaller than, at and past the edges of the kernel's
+    15 x 4 x 4 tiles."""
+    net = LG.UNet(dims, seed=1)
+    p = torch.zeros(net.n_params)
+    c = torch.tensor([2.0 ** (i % 4 - 2) for i in range(16)])
+    layers = LG.unpack(p)  # views
+    layers[12][1][:], layers[13][1][:] = c, c.flip(0)  # inputs of layers 13 and 14
+    wo = torch.tensor([2.0 ** (i % 3) for i in range(16)])
+    layers[14][0][0, :, 1, 1, 1] = wo
+    net.set_params(p)
+    n = dims[0] * dims[1] * dims[2]
+    g = torch.Generator().manual_seed(n)
+    net.forward(torch.zeros(3 * n, device="cuda"))
+    gy = torch.randint(-2, 3, (n,), generator=g).float()
+    got = LG.unpack(net.backward(gy.cuda()).cpu())
+    vol = F.pad(gy.double().view(dims[2], dims[1], dims[0]), (1, 1, 1, 1, 1, 1))
+    # sum of gy over the points whose neighbour at tap (dz, dy, dx) lies in the grid
+    taps = torch.zeros(3, 3, 3, dtype=torch.float64)
+    inside = F.pad(torch.ones(dims[2], dims[1], dims[0], dtype=torch.float64), (1,) * 6)
+    for dz in range(3):
+        for dy in range(3):
+            for dx in range(3):
+                nb = torch.roll(inside, (1 - dz, 1 - dy, 1 - dx), (0, 1, 2))
+                taps[dz, dy, dx] = (vol * nb).sum()
+    assert torch.equal(got[14][0][0].double(), c.flip(0).double().view(16, 1, 1, 1) * taps)
+    assert torch.equal(got[14][1].double(), gy.double().sum().view(1))
+    assert torch.equal(got[13][0].double(), wo.double().view(16, 1, 1, 1, 1) *
+                       c.double().view(1, 16, 1, 1, 1) * taps)
+    assert torch.equal(got[13][1].double(), wo.double() * gy.double().sum())
