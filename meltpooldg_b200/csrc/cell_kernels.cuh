@@ -62,13 +62,6 @@ template <typename T> __device__ __forceinline__ void atomic_add(T *p, T v) { at
 template <int LAW> __host__ __device__ constexpr bool law_tdep() { return LAW == 1 || LAW == 2 || LAW == 5; }
 // laws that may need T_old (d(rho_cp)/dT (T_lin - T_old) / dt in the tangent)
 template <int LAW> __host__ __device__ constexpr bool law_told() { return LAW == 2 || LAW == 5; }
-// shared arrays per cell of the line-per-thread operator: u and its gradients, a temporary (Tq
-// doubles as it with T_lin), T_lin's values and gradients, T_old's values
-template <int LAW> __host__ __device__ constexpr int vmult_arrays()
-{
-  return law_tdep<LAW>() ? (law_told<LAW>() ? 9 : 8) : 5;
-}
-
 // a - 2 b (one operation)
 __device__ __forceinline__ float minus_twice(float a, float b) { return fmaf(-2.f, b, a); }
 __device__ __forceinline__ double minus_twice(double a, double b) { return fma(-2.0, b, a); }
@@ -313,6 +306,15 @@ __device__ __forceinline__ void geo_at(const GeoParams<T> &g, int64_t cell, int 
   }
 }
 
+// a x b
+template <typename T>
+__device__ __forceinline__ void cross(const T (&a)[3], const T (&b)[3], T (&c)[3])
+{
+  c[0] = a[1] * b[2] - a[2] * b[1];
+  c[1] = a[2] * b[0] - a[0] * b[2];
+  c[2] = a[0] * b[1] - a[1] * b[0];
+}
+
 template <int GEO, typename T>
 __device__ __forceinline__ void apply_G(const T G[6], T a, T b, T c, T &x, T &y, T &z)
 {
@@ -324,231 +326,6 @@ __device__ __forceinline__ void apply_G(const T G[6], T a, T b, T c, T &x, T &y,
     x = G[0] * a + G[1] * b + G[2] * c;
     y = G[1] * a + G[3] * b + G[4] * c;
     z = G[2] * a + G[4] * b + G[5] * c;
-  }
-}
-
-// L2 prefetch of the next batch of a line-per-thread kernel: this thread's x-line of each
-// given vector and, cooperatively over the block, the batch's contiguous per-cell blocks of
-// per-q data (nper values per q-point), so the next batch's gathers and q-point loads hit L2
-// instead of stalling on DRAM (the long-scoreboard stall of the q-point loop).
-template <int n, typename T>
-__device__ __forceinline__ void prefetch_next_batch(const MeshDims &d, int64_t n_cells,
-                                                    int64_t next_batch, int cl, int j, int k,
-                                                    const T *v0, const T *v1, const T *perq,
-                                                    int nper)
-{
-  constexpr int n3 = n * n * n, CPB = cells_per_block(n);
-  const int64_t first = next_batch * CPB;
-  if (first >= n_cells) return;
-  const int64_t ncell = first + cl;
-  if (ncell < n_cells) {
-    const int ncx = (int)(ncell % d.m[0]);
-    const int ncy = (int)((ncell / d.m[0]) % d.m[1]);
-    const int ncz = (int)(ncell / ((int64_t)d.m[0] * d.m[1]));
-    const int64_t nrow =
-      (int64_t)d.nd[0] * ((d.p * ncy + j) + (int64_t)d.nd[1] * (d.p * ncz + k)) + d.p * ncx;
-    for (const T *v : {v0, v1}) {
-      if (!v) continue;
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(v + nrow));
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(v + nrow + n - 1));
-    }
-  }
-  if (perq) {
-    const int64_t last = first + CPB < n_cells ? first + CPB : n_cells;
-    const char *g0 = reinterpret_cast<const char *>(perq + first * nper * n3);
-    const int64_t bytes = (last - first) * nper * n3 * (int64_t)sizeof(T);
-    for (int64_t off = (int64_t)threadIdx.x * 128; off < bytes; off += (int64_t)blockDim.x * 128)
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(g0 + off));
-  }
-}
-
-// ---------------------------------------------------------------------------
-// vmult: dst += J src (dst zeroed by the caller); optional src.dst dot
-// ---------------------------------------------------------------------------
-// PRE (deformed meshes): this batch's per-point geometry (7 values at each of the thread's n
-// points) is loaded into registers when the batch starts, so those loads are in flight during
-// the gather and the evaluation sweeps instead of stalling the quadrature-point loop.
-template <int n, typename T, int GEO, int LAW, bool PRE = false>
-__global__ void __launch_bounds__(block_threads(n)) k_vmult(CellArgs<T> a)
-{
-  constexpr int n2 = n * n, n3 = n2 * n, CPB = cells_per_block(n);
-  constexpr bool TDEP = law_tdep<LAW>();
-  static_assert(!PRE || GEO == 1, "the geometry preload is for per-point geometry");
-  // shared arrays per cell: the sweeps' temporaries alias arrays that are free at that time
-  // (gx, gy while values are interpolated, the gathered T_lin in gz, Tq after the q-point loop)
-  constexpr int NF = vmult_arrays<LAW>();
-  if (a.st && a.st->done) return;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T *sm = reinterpret_cast<T *>(smem_raw);
-  const int cl = threadIdx.x / n2, line = threadIdx.x % n2;
-  T *u = sm + cl * NF * n3, *gx = u + n3, *gy = u + 2 * n3, *gz = u + 3 * n3;
-  T *t1 = u + 4 * n3;  // integration temporary without the T_lin arrays
-  T *Tq = u + 4 * n3, *Tx = u + 5 * n3, *Ty = u + 6 * n3, *Tz = u + 7 * n3, *Toq = u + 8 * n3;
-  const MeshDims &d = a.d;
-  double dot = 0.0;
-  const int64_t n_batches = (a.n_cells + CPB - 1) / CPB;
-  for (int64_t batch = blockIdx.x; batch < n_batches; batch += gridDim.x) {
-    const int64_t cell = batch * CPB + cl;
-    const bool active = cell < a.n_cells;
-    const int64_t cc = active ? cell : 0;
-    const int cx = (int)(cc % d.m[0]);
-    const int cy = (int)((cc / d.m[0]) % d.m[1]);
-    const int cz = (int)(cc / ((int64_t)d.m[0] * d.m[1]));
-    const int j = line % n, k = line / n;
-    const int I0 = d.p * cx, J = d.p * cy + j, K = d.p * cz + k;
-    const int64_t row = (int64_t)d.nd[0] * (J + (int64_t)d.nd[1] * K) + I0;
-    T gpre[PRE ? n : 1][7];
-    T fpre[(PRE && LAW == 7) ? n : 1][4];
-    if (PRE) {
-      const T *gb = a.g.q + cc * 7 * n3 + line;
-#pragma unroll
-      for (int r = 0; r < n; ++r)
-#pragma unroll
-        for (int c = 0; c < 7; ++c) gpre[r][c] = __ldg(gb + c * n3 + n2 * r);
-      if (LAW == 7) {
-        const T *fb = a.cf + cc * 4 * n3 + line;
-#pragma unroll
-        for (int r = 0; r < n; ++r)
-#pragma unroll
-          for (int c = 0; c < 4; ++c) fpre[r][c] = __ldg(fb + c * n3 + n2 * r);
-      }
-    }
-    // the geometry, or the coefficient fields of LAW 4/5, dominate a batch's q-point loads
-    if (GEO == 1)
-      prefetch_next_batch<n>(d, a.n_cells, batch + gridDim.x, cl, j, k, a.src,
-                             TDEP ? a.Tl : nullptr, a.g.q, 7);
-    else
-      prefetch_next_batch<n>(d, a.n_cells, batch + gridDim.x, cl, j, k, a.src,
-                             TDEP ? a.Tl : nullptr, (LAW == 4 || LAW == 5) ? a.cf : nullptr, 5);
-    T xs[n];
-    gather_xline<n>(d, row, I0, J, K, true, a.src, xs, active);
-#pragma unroll
-    for (int i = 0; i < n; ++i) u[i + n * line] = xs[i];
-    if (TDEP) {
-      T xt[n];
-      if (law_told<LAW>() && a.m.need_told) {
-        gather_xline<n>(d, row, I0, J, K, false, a.To, xt, active);
-#pragma unroll
-        for (int i = 0; i < n; ++i) Tq[i + n * line] = xt[i];
-      }
-      gather_xline<n>(d, row, I0, J, K, false, a.Tl, xt, active);
-#pragma unroll
-      for (int i = 0; i < n; ++i) gz[i + n * line] = xt[i];
-    }
-    __syncthreads();
-    if (TDEP) {
-      // T_lin values + gradients: gz -> (S) -> Tq; old values first if needed
-      if (law_told<LAW>() && a.m.need_told) {
-        eval_values<n>(Tq, gx, gy, Toq, line);
-      }
-      eval_values<n>(gz, gx, gy, Tq, line);
-      eval_gradients<n>(Tq, Tx, Ty, Tz, line);
-    }
-    eval_values<n>(u, gx, gy, u, line);  // values overwrite the gathered nodal values
-    eval_gradients<n>(u, gx, gy, gz, line);
-    // quadrature-point operation (tangent_local_cell_operation)
-#pragma unroll
-    for (int r = 0; r < n; ++r) {
-      const int q = line + n2 * r;
-      const int qi = q % n, qj = (q / n) % n, qk = q / n2;
-      T jxw, G[6];
-      if (PRE) {
-        jxw = gpre[r][0];
-#pragma unroll
-        for (int c = 0; c < 6; ++c) G[c] = gpre[r][1 + c];
-      } else {
-        geo_at<n, GEO>(a.g, cc, qi, qj, qk, jxw, G);
-      }
-      T rhocp, kk, drhocp, dk;
-      const T uu = u[q];
-      T val, b0 = T(0), b1 = T(0), b2 = T(0);
-      if (LAW == 5) {
-        const T *cf = a.cf + cc * 5 * n3 + q;
-        mat_eval_w(a.m, Tq[q], __ldg(cf), rhocp, kk, drhocp, dk);
-        b0 = __ldg(cf + 2 * n3);
-        b1 = __ldg(cf + 3 * n3);
-        b2 = __ldg(cf + 4 * n3);
-      } else if (LAW == 4) {
-        const T *cf = a.cf + cc * 5 * n3 + q;
-        kk = __ldg(cf + n3);
-        rhocp = drhocp = dk = T(0);
-        val = a.m.idt * __ldg(cf) * uu + __ldg(cf + 2 * n3) * gx[q] + __ldg(cf + 3 * n3) * gy[q] +
-              __ldg(cf + 4 * n3) * gz[q];
-      } else if (LAW == 7) {
-        // linear-k tangent from its fields: k(T_lin) and k1 dT_lin/dxi_d at the point
-        T fk, fd[3];
-        if (PRE) {
-          fk = fpre[r][0];
-#pragma unroll
-          for (int c = 0; c < 3; ++c) fd[c] = fpre[r][1 + c];
-        } else {
-          const T *cf = a.cf + cc * 4 * n3 + q;
-          fk = __ldg(cf);
-#pragma unroll
-          for (int c = 0; c < 3; ++c) fd[c] = __ldg(cf + (1 + c) * n3);
-        }
-        kk = fk;
-        rhocp = a.m.rho_l * a.m.cp_l;
-        drhocp = dk = T(0);
-        b0 = fd[0];
-        b1 = fd[1];
-        b2 = fd[2];
-      } else {
-        mat_eval<LAW>(a.m, TDEP ? Tq[q] : T(0), rhocp, kk, drhocp, dk);
-      }
-      T cval = a.m.idt * rhocp;
-      T f0 = kk * gx[q], f1 = kk * gy[q], f2 = kk * gz[q];
-      if (LAW == 7) {
-        f0 += b0 * uu;
-        f1 += b1 * uu;
-        f2 += b2 * uu;
-      }
-      if (TDEP) {
-        if (law_told<LAW>() && a.m.need_told) cval += a.m.idt * drhocp * (Tq[q] - Toq[q]);
-        f0 += dk * Tx[q] * uu;
-        f1 += dk * Ty[q] * uu;
-        f2 += dk * Tz[q] * uu;
-      }
-      if (LAW == 5)  // rho_cp b.grad(u) + d(rho_cp)/dT (b.grad T) u, b = JxW J^-1 v
-        val = cval * uu * jxw + rhocp * (b0 * gx[q] + b1 * gy[q] + b2 * gz[q]) +
-              drhocp * (b0 * Tx[q] + b1 * Ty[q] + b2 * Tz[q]) * uu;
-      u[q] = (LAW == 4 || LAW == 5) ? val : cval * uu * jxw;
-      T F0, F1, F2;
-      apply_G<GEO>(G, f0, f1, f2, F0, F1, F2);
-      gx[q] = F0;
-      gy[q] = F1;
-      gz[q] = F2;
-    }
-    __syncthreads();
-    integrate<n>(u, gx, gy, gz, t1, line);
-    // scatter the x-line (skip constrained rows) and accumulate src.dst
-    if (active) {
-#pragma unroll
-      for (int i = 0; i < n; ++i) {
-        const T r = u[i + n * line];
-        if (!constrained(d, I0 + i, J, K)) atomic_add(a.dst + row + i, r);
-        dot += (double)xs[i] * (double)r;
-      }
-    }
-    __syncthreads();
-  }
-  if (a.fin != FIN_NONE) {
-    double v[1] = {dot}, tot[1];
-    if (grid_sum<1>(v, a.partials, a.counter, tot)) {
-      if (a.extra_dot) tot[0] += *a.extra_dot;
-      if (a.fin == FIN_STORE) {
-        *a.out = tot[0];
-      } else {
-        SolverState *s = a.st;
-        s->pAp = tot[0];
-        if (!(tot[0] > 0.0) || !isfinite(tot[0])) {
-          s->done = 2;
-          s->status = 5;  // breakdown
-        } else {
-          s->alpha = s->rz / tot[0];
-        }
-      }
-    }
   }
 }
 
@@ -1017,10 +794,6 @@ __global__ void __launch_bounds__(block_threads(n)) k_norm(CellArgs<double> a)
 }
 
 // shared-memory bytes of each kernel
-template <int n, typename T, int LAW> constexpr size_t smem_vmult()
-{
-  return sizeof(T) * cells_per_block(n) * vmult_arrays<LAW>() * n * n * n;
-}
 template <int n> constexpr size_t smem_rhs() { return sizeof(double) * cells_per_block(n) * 9 * n * n * n; }
 template <int n> constexpr size_t smem_diag() { return sizeof(double) * cells_per_block(n) * 16 * n * n * n; }
 template <int n> constexpr size_t smem_norm() { return sizeof(double) * cells_per_block(n) * 4 * n * n * n; }

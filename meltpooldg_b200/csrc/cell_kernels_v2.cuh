@@ -317,15 +317,6 @@ __device__ __forceinline__ void load_map(const MeshDims &d, const double *__rest
     map[(3 * kMapH + e) * stride] = exyz;
   }
 }
-// a x b
-template <typename T>
-__device__ __forceinline__ void cross(const T (&a)[3], const T (&b)[3], T (&c)[3])
-{
-  c[0] = a[1] * b[2] - a[2] * b[1];
-  c[1] = a[2] * b[0] - a[0] * b[2];
-  c[2] = a[0] * b[1] - a[1] * b[0];
-}
-
 // Blocks per SM that the register allocator is held to. Without a bound it hoists the row loads
 // and the scatter's addresses until half as many warps fit (FP32 Picard p = 3: 195 registers, 8
 // warps, 0.96 ms against 0.52 ms with 128 registers, 16 warps, on 128^3 cells); a tighter bound

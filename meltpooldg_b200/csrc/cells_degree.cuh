@@ -5,6 +5,7 @@
 #pragma once
 
 #include "cell_kernels.cuh"
+#include "cell_kernels_lines.cuh"
 #include "cell_kernels_v2.cuh"
 #include "cell_kernels_f2.cuh"
 #include "cell_kernels_tc.cuh"
@@ -47,18 +48,6 @@ static inline bool fp32_packed()
   return on != 0;
 }
 
-// Line-per-thread operator on deformed meshes: the batch's per-point geometry
-// preloaded into registers (default) or loaded in the quadrature-point loop
-// (MPDG_GEO_PRELOAD=0); both compute the same operator.
-static inline bool geo_preload()
-{
-  static const int on = [] {
-    const char *e = getenv("MPDG_GEO_PRELOAD");
-    return (e && e[0] == '0') ? 0 : 1;
-  }();
-  return on != 0;
-}
-
 template <int n>
 struct DegreeOps {
   static constexpr int CPB = cells_per_block(n);
@@ -75,14 +64,20 @@ struct DegreeOps {
     cudaMemcpyToSymbol(c_w_f, wf, sizeof(float) * kWTabSize);
   }
 
-  // register-resident kernel where a cell's planes fit the register file (FP64 at
-  // p = 4 spills 64-750 bytes there and measured no faster than the line-per-thread
-  // kernel on the deformed mesh, so it stays on the latter); the three-phase / transport
-  // law with temperature dependence (LAW 5) runs the line-per-thread kernel
+  // register-resident kernel where a cell's planes fit the register file; the three-phase /
+  // transport law with temperature dependence (LAW 5) runs the line kernel
   template <typename T, int LAW = 0>
   static constexpr bool use_v2()
   {
     return LAW != 5 && (sizeof(T) == 8 ? n <= 4 : n <= 5);
+  }
+  // the operator alone also with the constant law on a uniform box up to p = 5, which spills but
+  // needs no per-point data (FP64 p = 4 on 64^3 cells 0.30 against 0.42 ms on lines, p = 5 on 53^3
+  // 0.43 against 0.50 ms; FP32 p = 5 0.23 against 0.26 ms)
+  template <typename T, int GEO, int LAW>
+  static constexpr bool vmult_v2()
+  {
+    return use_v2<T, LAW>() || (GEO == 0 && LAW == 0 && n <= 6);
   }
 
   template <typename T, int GEO, int LAW>
@@ -100,35 +95,39 @@ struct DegreeOps {
         return cudaGetLastError();
       }
     }
-    if constexpr (use_v2<T, LAW>()) {
-      static int cache2 = 0;
-      // deformed FP64: the geometry from the cell's vertices (p >= 2) instead of the stored one
-      constexpr int G = v2_geometry<n, T, GEO>();
-      auto k2 = k_vmult2<n, T, G, LAW>;
-      const size_t smem2 = v2_smem<n, T, LAW, G>();
-      const int64_t ng = (a.n_cells + v2_cells_per_warp<n>() - 1) / v2_cells_per_warp<n>();
-      const int g2 = persistent_grid(k2, 32 * kV2Warps, smem2, (ng + kV2Warps - 1) / kV2Warps, sm,
-                                     &cache2);
-      k2<<<g2, 32 * kV2Warps, smem2, s>>>(a);
-      return cudaGetLastError();
-    } else {
-      const size_t smem = smem_vmult<n, T, LAW>();
-      const int64_t nb = (a.n_cells + CPB - 1) / CPB;
-      if constexpr (GEO == 1) {
-        if (geo_preload()) {
-          static int cachep = 0;
-          auto kp = k_vmult<n, T, GEO, LAW, true>;
-          const int g = persistent_grid(kp, THREADS, smem, nb, sm, &cachep);
-          kp<<<g, THREADS, smem, s>>>(a);
-          return cudaGetLastError();
-        }
-      }
-      static int cache = 0;
-      auto k = k_vmult<n, T, GEO, LAW>;
-      const int g = persistent_grid(k, THREADS, smem, nb, sm, &cache);
-      k<<<g, THREADS, smem, s>>>(a);
-      return cudaGetLastError();
+    // at p = 5 only where the cells fill a round of the grid (8 warps per SM): below that the time
+    // is one cell group's latency, which is longer with the spills (729 cells FP64 16.4 us, the
+    // line kernel 12.3)
+    const bool fills = n < 6 || a.n_cells >= (int64_t)sm * 8 * v2_cells_per_warp<n>();
+    if constexpr (vmult_v2<T, GEO, LAW>()) {
+      if (fills) return vmult_planes<T, GEO, LAW>(a, s, sm);
     }
+    if constexpr (!vmult_v2<T, GEO, LAW>() || n == 6) return vmult_lines<T, GEO, LAW>(a, s, sm);
+    return cudaErrorNotSupported;  // (not reached: fills is true below n = 6)
+  }
+  template <typename T, int GEO, int LAW>
+  static cudaError_t vmult_planes(const CellArgs<T> &a, cudaStream_t s, int sm)
+  {
+    static int cache2 = 0;
+    // deformed FP64: the geometry from the cell's vertices (p >= 2) instead of the stored one
+    constexpr int G = v2_geometry<n, T, GEO>();
+    auto k2 = k_vmult2<n, T, G, LAW>;
+    const size_t smem2 = v2_smem<n, T, LAW, G>();
+    const int64_t ng = (a.n_cells + v2_cells_per_warp<n>() - 1) / v2_cells_per_warp<n>();
+    const int g2 = persistent_grid(k2, 32 * kV2Warps, smem2, (ng + kV2Warps - 1) / kV2Warps, sm,
+                                   &cache2);
+    k2<<<g2, 32 * kV2Warps, smem2, s>>>(a);
+    return cudaGetLastError();
+  }
+  template <typename T, int GEO, int LAW>
+  static cudaError_t vmult_lines(const CellArgs<T> &a, cudaStream_t s, int sm)
+  {
+    static int cache = 0;
+    auto k = k_vmult_lines<n, T, ln_geometry<T, GEO, LAW>(), LAW>;
+    constexpr size_t smem = ln_smem<n, T>();
+    const int g = persistent_grid(k, THREADS, smem, (a.n_cells + CPB - 1) / CPB, sm, &cache);
+    k<<<g, THREADS, smem, s>>>(a);
+    return cudaGetLastError();
   }
   template <typename T>
   static cudaError_t vmult(const CellArgs<T> &a, int geo, int law, cudaStream_t s, int sm)

@@ -10,6 +10,7 @@
 //   DT  its transpose
 //   PT  (S o S)^T, QT = (Sd o Sd)^T, RT = (S o Sd)^T, with Sd = D S: the
 //       element-wise products that give the closed-form diagonal
+//   G   derivative of the nodal basis at the Gauss points, Sd = D S; GT its transpose
 // All of them are centro-(anti)symmetric: A[n-1-o][n-1-l] = sym * A[o][l].
 #pragma once
 
@@ -25,9 +26,14 @@
 namespace mpdg {
 
 constexpr int kMaxN = 7;
-enum MatKind { kS = 0, kST = 1, kD = 2, kDT = 3, kPT = 4, kQT = 5, kRT = 6, kNumKinds = 7 };
+enum MatKind {
+  kS = 0, kST = 1, kD = 2, kDT = 3, kPT = 4, kQT = 5, kRT = 6, kG = 7, kGT = 8, kNumKinds = 9
+};
 
-MPDG_HD constexpr int kind_sym(int kind) { return (kind == kD || kind == kDT || kind == kRT) ? -1 : 1; }
+MPDG_HD constexpr int kind_sym(int kind)
+{
+  return (kind == kD || kind == kDT || kind == kRT || kind == kG || kind == kGT) ? -1 : 1;
+}
 
 // Per (n, kind) block: ae[n][h], ao[n][h], mid[n] with h = n/2, then the matrix itself [n][n].
 MPDG_HD constexpr int tab_full(int n) { return 2 * n * (n / 2) + n; }
@@ -166,6 +172,8 @@ inline Tables1D make_tables(int n)
       t.A[kPT][a][b] = S[b][a] * S[b][a];
       t.A[kQT][a][b] = Sd[b][a] * Sd[b][a];
       t.A[kRT][a][b] = S[b][a] * Sd[b][a];
+      t.A[kG][a][b] = Sd[a][b];
+      t.A[kGT][a][b] = Sd[b][a];
     }
   return t;
 }

@@ -51,3 +51,26 @@ def test_operator_verbs(degree, cells, perturb, mask):
     assert rel(1.0 / g.inverse_diagonal_picard_f32(g.new_vector(torch.float32)),
                1.0 / o.inverse_diagonal(Tl, To, form=2)) <= TOL32
     assert rel(g.create_rhs(g.new_vector(), d["To"], d["q"]), o.create_rhs(Tl, To, q)) <= TOL64
+
+
+@pytest.mark.parametrize("degree,cells", [(4, (23, 29, 31)), (5, (1, 1, 1)), (5, (13, 17, 19)),
+                                          (6, (1, 3, 1)), (6, (11, 13, 17))])
+@pytest.mark.parametrize("perturb", [0.0, 0.2])
+@pytest.mark.parametrize("law", ["constant", "linear_k"])
+def test_high_degree_operator(degree, cells, perturb, law):
+    """The line kernel (and at p = 4, 5 the register-resident one with the constant law on a uniform
+    box) on one cell, on a batch that is partly empty and over several rounds of the grid."""
+    m = KT if law == "linear_k" else dict(law=0, rho=1.0, cp=1.0, k=1.0)
+    mask, dt = 0b010010, 1e-3
+    o = O.Oracle(degree, cells, perturb=perturb, seed=5, dirichlet_mask=mask)
+    o.set_material(O.material(**m), dt)
+    g = H.HeatDiffuseOperator(H.box_mesh(degree, cells, perturb=perturb, seed=5, dirichlet=(1, 4)))
+    g.set_material(H.material(**m))
+    g.reset_time_increment(dt)
+    rng = np.random.default_rng(degree)
+    src, Tl = rng.uniform(-1.0, 1.0, o.n_dofs), rng.uniform(0.0, 1.0, o.n_dofs)
+    Tld = torch.tensor(Tl, device="cuda")
+    g.set_linearization(Tld, Tld)
+    s, ref = torch.tensor(src, device="cuda"), o.vmult(src, Tl, Tl)
+    assert rel(g.vmult(g.new_vector(), s), ref) <= TOL64
+    assert rel(g.vmult(g.new_vector(torch.float32), s.float()), ref) <= TOL32 * 10
