@@ -645,11 +645,10 @@ __global__ void __launch_bounds__(block_threads(n)) k_coef_tangent(CellArgs<doub
 }
 
 // ---------------------------------------------------------------------------
-// Tangent fields of the linear-k law at the linearisation point, built once per
-// linearisation for the register-resident kernel's LAW 7: out[cell][4][n^3] =
-// {k_l + k1 T_lin, k1 grad_ref T_lin} (the 7 T_lin sweeps of every LAW 1 application).
+// Tangent fields of the linear-k law at the linearisation point, built once per linearisation for
+// LAW 7 (p >= 4; below, k_coef_lineark2): out[cell][4][n^3] = {k_l + k1 T_lin, k1 grad_ref T_lin}.
 // ---------------------------------------------------------------------------
-template <int n, int GEO>
+template <int n>
 __global__ void __launch_bounds__(block_threads(n)) k_coef_lineark(CellArgs<double> a, double *out)
 {
   using T = double;

@@ -874,6 +874,244 @@ __global__ void __launch_bounds__(32 * kV2Warps) k_diag_picard(CellArgs<float> a
   }
 }
 
+// a row of n values to global memory (as load_row reads it)
+template <int n>
+__device__ __forceinline__ void store_row(double *p, const double (&r)[n])
+{
+  if constexpr (n == 4) {
+    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(r[0]), "d"(r[1]),
+                 "d"(r[2]), "d"(r[3])
+                 : "memory");
+  } else if constexpr (n == 2) {
+    *reinterpret_cast<double2 *>(p) = make_double2(r[0], r[1]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < n; ++i) p[i] = r[i];
+  }
+}
+
+// Tangent fields of the linear-k law at the linearisation point, built once per linearisation for
+// LAW 7: out[cell][4][n^3] = {k_l + k1 T_lin, k1 grad_ref T_lin}. On the planes of k_vmult2 with
+// 32-byte stores: bound by the 32 bytes a point that it writes (128^3 cells of FE_Q(3), 4.3 GB:
+// 1.59 ms on lines through shared memory, 1.14 ms here).
+template <int n>
+__global__ void __launch_bounds__(32 * kV2Warps, 4) k_coef_lineark2(CellArgs<double> a, double *out)
+{
+  using T = double;
+  constexpr int CW = v2_cells_per_warp<n>(), CS = v2_cell_stride<n>(), npt = n * n * n;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int cw = lane / n, t = lane % n;
+  const bool lane_ok = cw < CW;
+  T *wbuf = reinterpret_cast<T *>(smem_raw) + (size_t)warp * 2 * (CW + 1) * CS;
+  T *bufA = wbuf + cw * CS, *bufB = wbuf + (CW + 1) * CS + cw * CS;
+  const MeshDims &d = a.d;
+  const int64_t rs = d.nd[0], ps = (int64_t)d.nd[0] * d.nd[1];
+  const int64_t stride = (int64_t)gridDim.x * kV2Warps * CW;
+  const int64_t first = ((int64_t)blockIdx.x * kV2Warps + warp) * CW;  // the warp's first cell
+  CellWalk at(d, first + cw, stride, a.n_cells);
+  for (int64_t head = first; head < a.n_cells; head += stride) {
+    const int64_t cell = head + cw;
+    const bool active = lane_ok && cell < a.n_cells;
+    const int64_t cc = active ? cell : 0;
+    const int I = d.p * at.x + t, J0 = d.p * at.y, K0 = d.p * at.z;
+    const int64_t base = I + rs * J0 + ps * K0;
+    at.advance(d);
+    T Q[n][n], Dz[n][n], Tq[n][n], Tz[n][n], Ty[n][n];
+    gather_column<n>(a.Tl, base, rs, ps, Q, active);
+    psweep_b<n, kS, false>(Q, Q);
+    psweep_a<n, kS, false>(Q, Q);
+    psweep_a<n, kD, false>(Q, Dz);
+    x_to_z2<n>(Q, Dz, Tq, Tz, bufA, bufB, t);
+    psweep_b<n, kS, false>(Tq, Tq);
+    psweep_b<n, kS, false>(Tz, Tz);
+    psweep_a<n, kD, false>(Tq, Ty);
+    if (active) {
+#pragma unroll
+      for (int j = 0; j < n; ++j) {
+        T Tx[n];
+        contract_row<n, kD, false>(Tq[j], Tx);
+        T *o = out + cc * 4 * npt + t * (n * n) + n * j;
+#pragma unroll
+        for (int i = 0; i < n; ++i) {
+          Tq[j][i] = a.m.k_l + a.m.k1 * Tq[j][i];
+          Tx[i] *= a.m.k1;
+          Ty[j][i] *= a.m.k1;
+          Tz[j][i] *= a.m.k1;
+        }
+        store_row<n>(o, Tq[j]);
+        store_row<n>(o + npt, Tx);
+        store_row<n>(o + 2 * npt, Ty[j]);
+        store_row<n>(o + 3 * npt, Tz[j]);
+      }
+    }
+  }
+}
+
+// Y[a][i] += A[a][q] x[i] for the transposed product matrix of `kind` and the row q
+template <int n, int kind>
+__device__ __forceinline__ void add_outer(int q, const double (&x)[n], double (&Y)[n][n])
+{
+  constexpr int full = tab_off(n, kind) + tab_full(n);
+#pragma unroll
+  for (int a = 0; a < n; ++a)
+#pragma unroll
+    for (int i = 0; i < n; ++i) Y[a][i] = fma(ctab<double>(full + a * n + q), x[i], Y[a][i]);
+}
+
+// FP64 diagonal of the operator (k_diag's closed form) for the constant and the linear-k law on
+// register planes: with P = S o S, Q = D o D, R = S o D (transposed tables) the x-contractions run
+// within a row of the quadrature plane, the y-contractions add each finished row to the three planes
+// that z contracts,
+//   Y_P = P_y (P_x C0 + Q_x Gxx + R_x Bx) + Q_y P_x Gyy + R_y (R_x Gxy + P_x By)
+//   Y_Q = P_y P_x Gzz      Y_R = P_y (R_x Gxz + P_x Bz) + R_y P_x Gyz
+//   W = P_z Y_P + Q_z Y_Q + R_z Y_R
+// so that no coefficient plane is kept (k_diag keeps ten in shared memory and takes 28 barriers a
+// batch; the inverse diagonal on 64^3 cells of FE_Q(3) k(T) 673 -> 183 us, deformed 768 -> 366).
+template <int n, int GEO, int LAW>
+__global__ void __launch_bounds__(32 * kV2Warps, 4) k_diag2(CellArgs<double> a)
+{
+  static_assert(LAW == 0 || LAW == 1, "constant rho*cp laws");
+  using T = double;
+  constexpr int CW = v2_cells_per_warp<n>(), CS = v2_cell_stride<n>(), npt = n * n * n;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int cw = lane / n, t = lane % n;
+  const bool lane_ok = cw < CW;
+  constexpr size_t kWarp = 2 * (CW + 1) * CS + (LAW == 1 ? 3 * n * n * 32 : 0);
+  T *wbuf = reinterpret_cast<T *>(smem_raw) + (size_t)warp * kWarp;
+  T *bufA = wbuf + cw * CS, *bufB = wbuf + (CW + 1) * CS + cw * CS;
+  T *keep = wbuf + 2 * (CW + 1) * CS + lane;  // LAW 1: T_lin, d/dy, d/dz, thread-private columns
+  const T cval = a.m.idt * (a.m.rho_l * a.m.cp_l);
+  const MeshDims &d = a.d;
+  const int64_t rs = d.nd[0], ps = (int64_t)d.nd[0] * d.nd[1];
+  const int64_t stride = (int64_t)gridDim.x * kV2Warps * CW;
+  const int64_t first = ((int64_t)blockIdx.x * kV2Warps + warp) * CW;  // the warp's first cell
+  CellWalk at(d, first + cw, stride, a.n_cells);
+  for (int64_t head = first; head < a.n_cells; head += stride) {
+    const int64_t cell = head + cw;
+    const bool active = lane_ok && cell < a.n_cells;
+    const int64_t cc = active ? cell : 0;
+    const int I = d.p * at.x + t, J0 = d.p * at.y, K0 = d.p * at.z;
+    const int64_t base = I + rs * J0 + ps * K0;
+    at.advance(d);
+    const ColumnMask cm(d, I, J0, K0, d.p);
+    if constexpr (LAW == 1) {
+      T Q[n][n], Dz[n][n], Tq[n][n], Tz[n][n], Ty[n][n];
+      gather_column<n>(a.Tl, base, rs, ps, Q, active);
+      psweep_b<n, kS, false>(Q, Q);
+      psweep_a<n, kS, false>(Q, Q);
+      psweep_a<n, kD, false>(Q, Dz);
+      x_to_z2<n>(Q, Dz, Tq, Tz, bufA, bufB, t);
+      psweep_b<n, kS, false>(Tq, Tq);
+      psweep_b<n, kS, false>(Tz, Tz);
+      psweep_a<n, kD, false>(Tq, Ty);
+#pragma unroll
+      for (int j = 0; j < n; ++j)
+#pragma unroll
+        for (int i = 0; i < n; ++i) {
+          keep[(0 * n * n + j * n + i) * 32] = Tq[j][i];
+          keep[(1 * n * n + j * n + i) * 32] = Ty[j][i];
+          keep[(2 * n * n + j * n + i) * 32] = Tz[j][i];
+        }
+    }
+    T YP[n][n], YQ[n][n], YR[n][n];
+#pragma unroll
+    for (int j = 0; j < n; ++j)
+#pragma unroll
+      for (int i = 0; i < n; ++i) YP[j][i] = YQ[j][i] = YR[j][i] = T(0);
+#pragma unroll
+    for (int j = 0; j < n; ++j) {
+      T C0[n], G[6][n], Tq[n], Tx[n], r[n];
+      if constexpr (GEO == 1) {
+        const T *gb = a.g.q + cc * 7 * npt + t * (n * n) + n * j;
+        load_row<n>(gb, C0);
+#pragma unroll
+        for (int f = 0; f < 6; ++f) load_row<n>(gb + (1 + f) * npt, G[f]);
+      } else {
+#pragma unroll
+        for (int i = 0; i < n; ++i) {
+          T g[6];
+          geo_at<n, GEO>(a.g, cc, i, j, t, C0[i], g);
+#pragma unroll
+          for (int f = 0; f < 6; ++f) G[f][i] = g[f];
+        }
+      }
+      if constexpr (LAW == 1) {
+#pragma unroll
+        for (int i = 0; i < n; ++i) Tq[i] = keep[(j * n + i) * 32];
+        contract_row<n, kD, false>(Tq, Tx);
+      }
+      T B[3][n];
+#pragma unroll
+      for (int i = 0; i < n; ++i) {
+        T rhocp, kk, drhocp, dk;
+        mat_eval<LAW>(a.m, LAW == 1 ? Tq[i] : T(0), rhocp, kk, drhocp, dk);
+        C0[i] *= cval;
+        if constexpr (LAW == 1) {
+          const T Ty = keep[(n * n + j * n + i) * 32], Tz = keep[(2 * n * n + j * n + i) * 32];
+          const T Gi[6] = {G[0][i], G[1][i], G[2][i], G[3][i], G[4][i], G[5][i]};
+          apply_G<GEO>(Gi, dk * Tx[i], dk * Ty, dk * Tz, B[0][i], B[1][i], B[2][i]);
+        }
+#pragma unroll
+        for (int f = 0; f < 6; ++f) G[f][i] *= kk;
+        G[1][i] *= T(2);
+        G[2][i] *= T(2);
+        G[4][i] *= T(2);
+      }
+      contract_row<n, kPT, false>(C0, r);
+      contract_row<n, kQT, true>(G[0], r);
+      if constexpr (LAW == 1) contract_row<n, kRT, true>(B[0], r);
+      add_outer<n, kPT>(j, r, YP);
+      contract_row<n, kPT, false>(G[3], r);
+      add_outer<n, kQT>(j, r, YP);
+      contract_row<n, kPT, false>(G[5], r);
+      add_outer<n, kPT>(j, r, YQ);
+      if constexpr (GEO == 1 || LAW == 1) {
+        if constexpr (GEO == 1) {
+          contract_row<n, kRT, false>(G[1], r);
+          if constexpr (LAW == 1) contract_row<n, kPT, true>(B[1], r);
+        } else {
+          contract_row<n, kPT, false>(B[1], r);
+        }
+        add_outer<n, kRT>(j, r, YP);
+        if constexpr (GEO == 1) {
+          contract_row<n, kRT, false>(G[2], r);
+          if constexpr (LAW == 1) contract_row<n, kPT, true>(B[2], r);
+        } else {
+          contract_row<n, kPT, false>(B[2], r);
+        }
+        add_outer<n, kPT>(j, r, YR);
+        if constexpr (GEO == 1) {
+          contract_row<n, kPT, false>(G[4], r);
+          add_outer<n, kRT>(j, r, YR);
+        }
+      }
+    }
+    T XP[n][n], XQ[n][n], W[n][n];
+    z_to_x2<n>(YP, YQ, XP, XQ, bufA, bufB, t);
+    psweep_a<n, kPT, false>(XP, W);
+    psweep_a<n, kQT, true>(XQ, W);
+    if constexpr (GEO == 1 || LAW == 1) {
+      z_to_x1<n>(YR, XP, bufA, t);
+      psweep_a<n, kRT, true>(XP, W);
+    }
+    if (active) {
+#pragma unroll
+      for (int k = 0; k < n; ++k)
+#pragma unroll
+        for (int j = 0; j < n; ++j)
+          if (!cm.template at<n>(j, k)) atomic_add(a.dst + base + (rs * j + ps * k), W[k][j]);
+    }
+  }
+}
+template <int n, int LAW> constexpr size_t diag2_smem()
+{
+  return sizeof(double) * kV2Warps *
+         ((size_t)2 * (v2_cells_per_warp<n>() + 1) * v2_cell_stride<n>() +
+          (LAW == 1 ? 3 * n * n * 32 : 0));
+}
+
 // create_rhs on register-resident planes for laws with constant rho*cp (0, 1):
 // dst += -R(T) = -sum_q [ (c (T - T_old) - q_h) phi_i JxW + k(T) grad T . G grad phi_i ]
 // with c = rho*cp / dt (rhs_cell_loop, heat_diffuse_operator.cpp:393-529). The value

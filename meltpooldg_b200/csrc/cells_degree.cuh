@@ -212,6 +212,22 @@ struct DegreeOps {
   template <int GEO, int LAW>
   static cudaError_t diag_t(const CellArgs<double> &a, cudaStream_t s, int sm)
   {
+    if constexpr (use_v2<double>() && (LAW == 0 || LAW == 1)) {
+      static int cache2 = 0;
+      auto k2 = k_diag2<n, GEO, LAW>;
+      constexpr size_t smem2 = diag2_smem<n, LAW>();
+      const int64_t ng = (a.n_cells + v2_cells_per_warp<n>() - 1) / v2_cells_per_warp<n>();
+      const int g2 = persistent_grid(k2, 32 * kV2Warps, smem2, (ng + kV2Warps - 1) / kV2Warps, sm,
+                                     &cache2);
+      k2<<<g2, 32 * kV2Warps, smem2, s>>>(a);
+      return cudaGetLastError();
+    } else {
+      return diag_lines<GEO, LAW>(a, s, sm);
+    }
+  }
+  template <int GEO, int LAW>
+  static cudaError_t diag_lines(const CellArgs<double> &a, cudaStream_t s, int sm)
+  {
     static int cache = 0;
     auto k = k_diag<n, GEO, LAW>;
     const size_t smem = smem_diag<n>();
@@ -334,20 +350,24 @@ struct DegreeOps {
   {
     return geo == 0 ? coef_tangent_t<0>(a, out, s, sm) : coef_tangent_t<1>(a, out, s, sm);
   }
-  template <int GEO>
-  static cudaError_t coef_lineark_t(const CellArgs<double> &a, double *out, cudaStream_t s, int sm)
+  static cudaError_t coef_lineark(const CellArgs<double> &a, double *out, cudaStream_t s, int sm)
   {
     static int cache = 0;
-    auto k = k_coef_lineark<n, GEO>;
-    const size_t smem = smem_coef_lineark<n>();
-    const int g = persistent_grid(k, THREADS, smem, (a.n_cells + CPB - 1) / CPB, sm, &cache);
-    k<<<g, THREADS, smem, s>>>(a, out);
+    if constexpr (use_v2<double>()) {
+      auto k = k_coef_lineark2<n>;
+      constexpr size_t smem =
+        sizeof(double) * kV2Warps * 2 * (v2_cells_per_warp<n>() + 1) * v2_cell_stride<n>();
+      const int64_t ng = (a.n_cells + v2_cells_per_warp<n>() - 1) / v2_cells_per_warp<n>();
+      const int g = persistent_grid(k, 32 * kV2Warps, smem, (ng + kV2Warps - 1) / kV2Warps, sm,
+                                    &cache);
+      k<<<g, 32 * kV2Warps, smem, s>>>(a, out);
+    } else {
+      auto k = k_coef_lineark<n>;
+      const size_t smem = smem_coef_lineark<n>();
+      const int g = persistent_grid(k, THREADS, smem, (a.n_cells + CPB - 1) / CPB, sm, &cache);
+      k<<<g, THREADS, smem, s>>>(a, out);
+    }
     return cudaGetLastError();
-  }
-  static cudaError_t coef_lineark(const CellArgs<double> &a, double *out, int geo, cudaStream_t s,
-                                  int sm)
-  {
-    return geo == 0 ? coef_lineark_t<0>(a, out, s, sm) : coef_lineark_t<1>(a, out, s, sm);
   }
   static cudaError_t field_values(const CellArgs<double> &a, const double *H, const double *vel,
                                   int64_t n_dofs, double *cf, cudaStream_t s, int sm)

@@ -26,7 +26,7 @@ struct DegreeTable {
   cudaError_t (*field_values)(const CellArgs<double> &, const double *H, const double *vel,
                               int64_t n_dofs, double *cf, cudaStream_t, int sm) = nullptr;
   // linear-k tangent fields at a.Tl (4 per point, FP64)
-  cudaError_t (*coef_lineark)(const CellArgs<double> &, double *out, int geo, cudaStream_t,
+  cudaError_t (*coef_lineark)(const CellArgs<double> &, double *out, cudaStream_t,
                               int sm) = nullptr;
   // the register-resident operator kernel exists for this degree (FP64 / FP32)
   bool v2_d = false, v2_f = false;

@@ -1551,7 +1551,7 @@ static int ensure_lineark(mpdg_heat *h)
   CellArgs<double> a = cell_args<double>(h);
   a.g.q = h->geoq;
   a.Tl = h->T_lin;
-  CU(h->tab.coef_lineark(a, h->tk, h->geo, h->stream, h->sm_count));
+  CU(h->tab.coef_lineark(a, h->tk, h->stream, h->sm_count));
   ++h->launches;
   h->tk_dirty = false;
   return MPDG_OK;
