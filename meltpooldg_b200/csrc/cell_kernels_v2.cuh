@@ -38,6 +38,11 @@ template <int LAW> __host__ __device__ constexpr int v2_ncoef()
   return (LAW == 1) ? 4 : (LAW == 2 ? 5 : (LAW == 8 ? 1 : 0));
 }
 constexpr int kV2Warps = 2;  // warps per CTA
+// LAW 7's fields per point on register planes: k1 T_lin and k1 dT_lin/dzeta. (The line kernel reads
+// four, {k(T_lin), k1 grad_ref T_lin}.) Storing all four took 1.35 ms per application on 128^3 cells
+// of FE_Q(3), 5.6 GB; these two and the derivatives along the plane 1.25 ms, 3.4 GB (p = 2 0.59 ->
+// 0.51 ms, p = 1 on 160^3 0.30 -> 0.25 ms).
+constexpr int kTanFields2 = 2;
 template <int n> __host__ __device__ constexpr bool v2_map_shared() { return n >= 4; }
 template <int n, typename T, int LAW, int GEO = 0>
 __host__ __device__ constexpr size_t v2_smem_per_warp()
@@ -421,7 +426,7 @@ __global__ void __launch_bounds__(32 * kV2Warps, (v2_min_blocks<n, T, GEO, LAW>(
             asm volatile("prefetch.global.L2 [%0];" ::"l"(kq + off));
         }
         if (LAW == 4 || LAW == 6 || LAW == 7) {
-          constexpr int nf = LAW == 4 ? 5 : (LAW == 6 ? 8 : 4);
+          constexpr int nf = LAW == 4 ? 5 : (LAW == 6 ? 8 : kTanFields2);
           constexpr int bytes = nf * npt * (int)sizeof(T);
           const char *cf = reinterpret_cast<const char *>(a.cf + ncell * nf * npt);
           for (int off = t * 128; off < bytes; off += n * 128)
@@ -506,6 +511,13 @@ __global__ void __launch_bounds__(32 * kV2Warps, (v2_min_blocks<n, T, GEO, LAW>(
     T Uy[n][n];
     psweep_a<n, kD, false>(U, Uy);
 
+    T t0[LAW == 7 ? n : 1][LAW == 7 ? n : 1];  // LAW 7: k1 T_lin on the plane
+    if constexpr (LAW == 7) {
+#pragma unroll
+      for (int j = 0; j < n; ++j)
+        load_row<n>(a.cf + cc * kTanFields2 * npt + t * (n * n) + n * j, t0[j]);
+    }
+
     // ---- quadrature-point operation (tangent_local_cell_operation), row by row: row j of U
     // turns into val + D_x^T f_x, those of Uy and Uz into f_y and f_z
 #pragma unroll
@@ -534,7 +546,19 @@ __global__ void __launch_bounds__(32 * kV2Warps, (v2_min_blocks<n, T, GEO, LAW>(
       // coefficient rows of the field laws
       constexpr int NC = LAW == 4 ? 5 : (LAW == 6 ? 8 : (LAW == 7 ? 4 : 1));
       T c[NC][n];
-      if constexpr (LAW == 4 || LAW == 6 || LAW == 7) {
+      if constexpr (LAW == 7) {
+        // k1 T_lin of the row (c[0]) and its gradient: d/dx within the row, d/dy down the plane
+        contract_row<n, kD, false>(t0[j], c[1]);
+#pragma unroll
+        for (int i = 0; i < n; ++i) {
+          constexpr int full = tab_off(n, kD) + tab_full(n);
+          c[0][i] = a.m.k_l + t0[j][i];
+          c[2][i] = ctab<T>(full + j * n) * t0[0][i];
+#pragma unroll
+          for (int l = 1; l < n; ++l) c[2][i] = fma(ctab<T>(full + j * n + l), t0[l][i], c[2][i]);
+        }
+        load_row<n>(a.cf + (cc * kTanFields2 + 1) * npt + q0, c[3]);
+      } else if constexpr (LAW == 4 || LAW == 6) {
         const T *cf = a.cf + cc * NC * npt + q0;
 #pragma unroll
         for (int f = 0; f < NC; ++f) load_row<n>(cf + f * npt, c[f]);
@@ -891,9 +915,9 @@ __device__ __forceinline__ void store_row(double *p, const double (&r)[n])
 }
 
 // Tangent fields of the linear-k law at the linearisation point, built once per linearisation for
-// LAW 7: out[cell][4][n^3] = {k_l + k1 T_lin, k1 grad_ref T_lin}. On the planes of k_vmult2 with
-// 32-byte stores: bound by the 32 bytes a point that it writes (128^3 cells of FE_Q(3), 4.3 GB:
-// 1.59 ms on lines through shared memory, 1.14 ms here).
+// LAW 7: out[cell][2][n^3] = {k1 T_lin, k1 dT_lin/dzeta} (k_vmult2 forms the other two derivatives
+// on its planes). On the planes of k_vmult2 with 32-byte stores (128^3 cells of FE_Q(3): four
+// fields on lines through shared memory 1.59 ms, on planes 1.14 ms, these two 0.63 ms).
 template <int n>
 __global__ void __launch_bounds__(32 * kV2Warps, 4) k_coef_lineark2(CellArgs<double> a, double *out)
 {
@@ -917,7 +941,7 @@ __global__ void __launch_bounds__(32 * kV2Warps, 4) k_coef_lineark2(CellArgs<dou
     const int I = d.p * at.x + t, J0 = d.p * at.y, K0 = d.p * at.z;
     const int64_t base = I + rs * J0 + ps * K0;
     at.advance(d);
-    T Q[n][n], Dz[n][n], Tq[n][n], Tz[n][n], Ty[n][n];
+    T Q[n][n], Dz[n][n], Tq[n][n], Tz[n][n];
     gather_column<n>(a.Tl, base, rs, ps, Q, active);
     psweep_b<n, kS, false>(Q, Q);
     psweep_a<n, kS, false>(Q, Q);
@@ -925,24 +949,17 @@ __global__ void __launch_bounds__(32 * kV2Warps, 4) k_coef_lineark2(CellArgs<dou
     x_to_z2<n>(Q, Dz, Tq, Tz, bufA, bufB, t);
     psweep_b<n, kS, false>(Tq, Tq);
     psweep_b<n, kS, false>(Tz, Tz);
-    psweep_a<n, kD, false>(Tq, Ty);
     if (active) {
 #pragma unroll
       for (int j = 0; j < n; ++j) {
-        T Tx[n];
-        contract_row<n, kD, false>(Tq[j], Tx);
-        T *o = out + cc * 4 * npt + t * (n * n) + n * j;
+        T *o = out + cc * kTanFields2 * npt + t * (n * n) + n * j;
 #pragma unroll
         for (int i = 0; i < n; ++i) {
-          Tq[j][i] = a.m.k_l + a.m.k1 * Tq[j][i];
-          Tx[i] *= a.m.k1;
-          Ty[j][i] *= a.m.k1;
+          Tq[j][i] *= a.m.k1;
           Tz[j][i] *= a.m.k1;
         }
         store_row<n>(o, Tq[j]);
-        store_row<n>(o + npt, Tx);
-        store_row<n>(o + 2 * npt, Ty[j]);
-        store_row<n>(o + 3 * npt, Tz[j]);
+        store_row<n>(o + npt, Tz[j]);
       }
     }
   }

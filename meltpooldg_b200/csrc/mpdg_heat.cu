@@ -1547,7 +1547,7 @@ static bool tangent_fields_lpt(int p)
 static int ensure_lineark(mpdg_heat *h)
 {
   if (!h->tk_dirty) return MPDG_OK;
-  TRY(dvec(h, &h->tk, h->n_cells * 4 * h->npt));
+  TRY(dvec(h, &h->tk, h->n_cells * (h->tab.v2_d ? 2 : 4) * h->npt));  // (fields per point)
   CellArgs<double> a = cell_args<double>(h);
   a.g.q = h->geoq;
   a.Tl = h->T_lin;
