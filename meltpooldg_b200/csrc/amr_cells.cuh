@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(32 * kV2Warps, 4)
 {
   using T = double;
   constexpr int CW = v2_cells_per_warp<n>(), CS = v2_cell_stride<n>(), npt = n * n * n;
-  if (cg && cg->done) return;
+  dependents_may_start();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int cw = lane / n, t = lane % n;
@@ -155,6 +155,8 @@ __global__ void __launch_bounds__(32 * kV2Warps, 4)
   T *coef = wbuf + 2 * (CW + 1) * CS;
   const T wt = cw_at<n, T>(w_off(n), t);
   double dot = 0.0;
+  wait_for_predecessor();
+  if (cg && cg->done) return;
   const int64_t stride = (int64_t)gridDim.x * kV2Warps * CW;
   for (int64_t head = ((int64_t)blockIdx.x * kV2Warps + warp) * CW; head < a.n_cells;
        head += stride) {
@@ -396,6 +398,8 @@ __global__ void k_amr_cg_update(int64_t n, const double *__restrict__ D,
                                 const double *__restrict__ Ap, double *r, AmrCg *cg,
                                 double *partials, unsigned *counter)
 {
+  dependents_may_start();
+  wait_for_predecessor();
   if (cg->done) return;
   const double alpha = cg->alpha;
   double v[2] = {0.0, 0.0};
@@ -430,6 +434,8 @@ __global__ void k_amr_cg_direction(int64_t n, const double *__restrict__ D,
                                    const double *__restrict__ r, double *x, double *p, double *Ap,
                                    const AmrCg *cg)
 {
+  dependents_may_start();
+  wait_for_predecessor();
   if (cg->done) return;
   const double alpha = cg->alpha, beta = cg->beta;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;

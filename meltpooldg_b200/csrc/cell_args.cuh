@@ -98,6 +98,7 @@ struct CellArgs {
   double *out;         // FIN_STORE destination
   const double *extra_dot;  // boundary-face part of src.dst, added at finalisation (nullable)
   int fin;
+  int dependent;  // launch_dependent (launch.cuh): a short kernel of a Krylov iteration
   SourceEval source;  // create_rhs: the laser source at the support points (source.on)
 };
 

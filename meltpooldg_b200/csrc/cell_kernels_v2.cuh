@@ -22,6 +22,7 @@
 #pragma once
 
 #include "cell_kernels.cuh"
+#include "launch.cuh"
 
 namespace mpdg {
 
@@ -362,7 +363,7 @@ __global__ void __launch_bounds__(32 * kV2Warps, (v2_min_blocks<n, T, GEO, LAW>(
   // T_lin (k is affine in T, so this is the conductivity field of LAW 3 without storing it)
   constexpr bool TDEP = LAW == 1 || LAW == 2;
   constexpr bool TLIN = TDEP || LAW == 8;
-  if (a.st && a.st->done) return;
+  dependents_may_start();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int cw = lane / n, t = lane % n;
@@ -386,6 +387,8 @@ __global__ void __launch_bounds__(32 * kV2Warps, (v2_min_blocks<n, T, GEO, LAW>(
   const int64_t stride = (int64_t)gridDim.x * kV2Warps * CW;
   const int64_t first = ((int64_t)blockIdx.x * kV2Warps + warp) * CW;  // the warp's first cell
   CellWalk at(d, first + cw, stride, a.n_cells);
+  wait_for_predecessor();
+  if (a.st && a.st->done) return;
   for (int64_t head = first; head < a.n_cells; head += stride) {
     const int64_t cell = head + cw;
     const bool active = lane_ok && cell < a.n_cells;

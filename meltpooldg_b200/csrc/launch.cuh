@@ -1,0 +1,39 @@
+// Programmatic dependent launch for the short kernels of a Krylov iteration: a kernel launched with
+// launch_dependent may start while its predecessor in the stream still runs (once every block of
+// that has called dependents_may_start), sets up, and waits in wait_for_predecessor until the
+// predecessor has completed and its writes are visible. Every such kernel waits before its first
+// access to data that another kernel writes, also on the way to an early return. Outside such a
+// launch both calls do nothing.
+#pragma once
+
+#include <cuda_runtime.h>
+
+namespace mpdg {
+
+__device__ __forceinline__ void wait_for_predecessor()
+{
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void dependents_may_start()
+{
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <typename... P, typename... A>
+cudaError_t launch_dependent(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem,
+                             cudaStream_t stream, const A &...args)
+{
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
+}  // namespace mpdg

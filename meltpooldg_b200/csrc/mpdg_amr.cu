@@ -946,7 +946,10 @@ void launch_apply(const AmrCellArgs &a, AmrCg *cg, double *partials, unsigned *c
   constexpr size_t smem = amr_smem<n, EVAL>();
   constexpr int cells = kV2Warps * v2_cells_per_warp<n>();
   const int g = resident_grid(k, 32 * kV2Warps, (a.n_cells + cells - 1) / cells, smem);
-  k<<<g, 32 * kV2Warps, smem>>>(a, cg, partials, counter);
+  if (cg)  // (an error is read by the caller's cudaGetLastError)
+    launch_dependent(k, g, 32 * kV2Warps, smem, (cudaStream_t)0, a, cg, partials, counter);
+  else
+    k<<<g, 32 * kV2Warps, smem>>>(a, cg, partials, counter);
 }
 template <int n> void launch_tfields(const AmrCellArgs &a, double *tf)
 {
@@ -1144,8 +1147,13 @@ int cg_impl(mpdg_amr *h, double *x, const double *b, const double *inv, const do
   for (;;) {
     for (int i = 0; i < kAmrChunk; ++i) {
       TRY_AMR(apply_cells(h, a, h->cg));
-      k_amr_cg_update<<<gr, 512>>>(N, inv, Ap, r, h->cg, h->partials, h->counter);
-      k_amr_cg_direction<<<g, 256>>>(N, inv, r, x, p, Ap, h->cg);
+      // (dependent launches: the kernels take 8 to 30 us)
+      cudaError_t e = launch_dependent(k_amr_cg_update, gr, 512, 0, (cudaStream_t)0, N, inv, Ap, r,
+                                       h->cg, h->partials, h->counter);
+      if (e == cudaSuccess)
+        e = launch_dependent(k_amr_cg_direction, g, 256, 0, (cudaStream_t)0, N, inv, r, x, p, Ap,
+                             h->cg);
+      if (e != cudaSuccess) return fail(MPDG_ERR_CUDA, cudaGetErrorString(e));
     }
     const cudaError_t e = cudaMemcpy(&st, h->cg, sizeof(st), cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return fail(MPDG_ERR_CUDA, cudaGetErrorString(e));

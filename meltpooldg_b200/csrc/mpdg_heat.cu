@@ -25,6 +25,7 @@
 #include "fe_tables.hpp"
 #include "material_law.cuh"
 #include "picard_tc_layout.hpp"
+#include "launch.cuh"
 #include "reduce.cuh"
 #include "source_eval.cuh"
 
@@ -655,6 +656,8 @@ __global__ void k_cg_update_xr(int64_t N, double *x, double *r, const double *__
                                const double *__restrict__ Ap, const double *__restrict__ D,
                                SolverState *st, double *partials, unsigned *counter)
 {
+  dependents_may_start();
+  wait_for_predecessor();
   if (st->done) return;
   const double alpha = st->alpha;
   double v[2] = {0.0, 0.0};
@@ -680,6 +683,8 @@ __global__ void k_cg_update_xr(int64_t N, double *x, double *r, const double *__
 __global__ void k_cg_update_p(int64_t N, const double *__restrict__ r, double *p, double *Ap,
                               const double *__restrict__ D, const SolverState *st)
 {
+  dependents_may_start();
+  wait_for_predecessor();
   if (st->done) return;
   const double beta = st->beta;
   GRID_STRIDE(i, N)
@@ -1645,7 +1650,7 @@ static int launch_faces(mpdg_heat *h, int op, T *dst, const T *src, const T *Tl,
 
 // dst += J src (FP64); fin/out/st select the fused src.dst reduction
 static int op_apply_d(mpdg_heat *h, double *dst, const double *src, int fin, double *out,
-                      SolverState *st)
+                      SolverState *st, bool dependent = false)
 {
   TRY(ensure_dt(h));
   TRY(ensure_lin(h));
@@ -1673,6 +1678,8 @@ static int op_apply_d(mpdg_heat *h, double *dst, const double *src, int fin, dou
   a.fin = fin;
   a.out = out;
   a.st = st;
+  // (the boundary faces' kernels between it and its predecessor are launched in stream order)
+  a.dependent = dependent && !h->timing && !any_faces(h);
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (h->timing) {
     e0 = take_event(h);
@@ -1927,17 +1934,23 @@ static int cg_jacobi(mpdg_heat *h, const mpdg_solver_params *prm, double *x, con
   CU(cudaGetLastError());
   TRY(poll(h));
   const double res0 = h->st_host->res0;
+  // The three kernels of an iteration are launched as dependents of one another: on a small mesh
+  // (FE_Q(2), 16^3 cells) each runs for a few microseconds, about what a launch's start costs. An
+  // iteration issued after convergence exits at once but still costs its launches, so the chunks
+  // between polls stay short (that mesh's solve: 970 us with plain launches and chunks that
+  // doubled up to 64, 661 us).
   int chunk = 4;
   while (!h->st_host->done) {
     for (int c = 0; c < chunk; ++c) {
-      TRY(op_apply_d(h, h->Ap, h->pv, FIN_CG_ALPHA, nullptr, h->st));
-      k_cg_update_xr<<<g, VT, 0, h->stream>>>(N, x, h->r, h->pv, h->Ap, D, h->st, h->partials,
-                                              h->counter); ++h->launches;
-      k_cg_update_p<<<g, VT, 0, h->stream>>>(N, h->r, h->pv, h->Ap, D, h->st); ++h->launches;
+      TRY(op_apply_d(h, h->Ap, h->pv, FIN_CG_ALPHA, nullptr, h->st, true));
+      CU(launch_dependent(k_cg_update_xr, g, VT, 0, h->stream, N, x, h->r, h->pv, h->Ap, D, h->st,
+                          h->partials, h->counter));
+      ++h->launches;
+      CU(launch_dependent(k_cg_update_p, g, VT, 0, h->stream, N, h->r, h->pv, h->Ap, D, h->st));
+      ++h->launches;
     }
-    CU(cudaGetLastError());
     TRY(poll(h));
-    chunk = std::min(chunk * 2, 64);
+    chunk = std::min(chunk * 2, 16);
   }
   if (stats) {
     stats->iterations = h->st_host->it;
