@@ -1391,10 +1391,12 @@ static int chunk_grid(const mpdg_heat *h, int64_t N)
 
 __global__ void k_zero16(int64_t n, uint4 *p)
 {
+  dependents_may_start();
   GRID_STRIDE(i, n) p[i] = make_uint4(0u, 0u, 0u, 0u);
 }
 __global__ void k_zero4(int64_t n, unsigned *p)
 {
+  dependents_may_start();
   GRID_STRIDE(i, n) p[i] = 0u;
 }
 
@@ -3368,7 +3370,7 @@ extern "C" int mpdg_heat_vmult(mpdg_heat *h, double *dst, const double *src)
   if (!h || !dst || !src) return fail(MPDG_ERR_INVALID_ARGUMENT, "null argument");
   CU(cudaSetDevice(h->device));
   CU(zero_async(h, dst, sizeof(double) * h->n_dofs, h->stream));
-  return op_apply_d(h, dst, src, FIN_NONE, nullptr, nullptr);
+  return op_apply_d(h, dst, src, FIN_NONE, nullptr, nullptr, true);
 }
 
 extern "C" int mpdg_heat_vmult_f32(mpdg_heat *h, float *dst, const float *src)

@@ -74,3 +74,30 @@ def test_high_degree_operator(degree, cells, perturb, law):
     s, ref = torch.tensor(src, device="cuda"), o.vmult(src, Tl, Tl)
     assert rel(g.vmult(g.new_vector(), s), ref) <= TOL64
     assert rel(g.vmult(g.new_vector(torch.float32), s.float()), ref) <= TOL32 * 10
+
+
+@pytest.mark.parametrize("degree,cells", [(2, (16, 16, 16)), (3, (1, 2, 1)), (4, (9, 9, 9))])
+def test_application_in_a_cuda_graph(degree, cells):
+    """op.vmult (a zero fill and a kernel launched as its dependent) recorded and replayed on new
+    operands, and repeated without a wait in between."""
+    op = H.HeatDiffuseOperator(H.box_mesh(degree, cells, dirichlet=("z-",)))
+    op.set_material(H.material())
+    op.reset_time_increment(1e-3)
+    x, y, z = (op.new_vector() for _ in range(3))
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        op.sync_stream()
+        op.vmult(y, x.uniform_())
+        side.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            op.vmult(y, x)
+            op.vmult(z, y)
+        x.uniform_()
+        graph.replay()
+    side.synchronize()
+    op.sync_stream()
+    ry = op.vmult(op.new_vector(), x)
+    rz = op.vmult(op.new_vector(), ry)
+    assert (y - ry).abs().max() <= 1e-13 * ry.abs().max()
+    assert (z - rz).abs().max() <= 1e-12 * rz.abs().max()
