@@ -1537,11 +1537,11 @@ static bool tangent_fields_enabled()
   return on != 0;
 }
 
-// line-per-thread kernel (FP64, p >= 4) on deformed meshes: the linear-k tangent from the
-// fields (preloaded with the geometry) instead of evaluating T_lin. The default at p = 4 and 6,
-// where it measured faster per application (3.84 -> 3.26 ms and 4.64 -> 4.00 ms at ~57 M DoFs)
-// and per production step with the fields' build included; at p = 5 its 200 registers make it
-// slower (4.23 -> 5.91 ms). MPDG_TANGENT_FIELDS_LPT=1 takes it at every degree, =0 at none.
+// Line kernel (FP64, p >= 4) on deformed meshes: the linear-k tangent from the fields instead of
+// evaluating T_lin, at p = 4 and 6. Per application the fields are faster at every degree (p = 4
+// 64^3 0.66 against 0.74 ms, p = 5 53^3 0.78 against 0.83, p = 6 45^3 0.80 against 0.85), but each
+// linearisation pays for building them, and p = 5 has not been measured in a solve.
+// MPDG_TANGENT_FIELDS_LPT=1 takes them at every degree, =0 at none.
 static bool tangent_fields_lpt(int p)
 {
   static const int mode = [] {
@@ -1667,8 +1667,8 @@ static int op_apply_d(mpdg_heat *h, double *dst, const double *src, int fin, dou
     law = 6;
   } else if (law == MPDG_LAW_LINEAR_K && h->tab.coef_lineark && tangent_fields_enabled() &&
              (h->tab.v2_d || (h->geo == 1 && tangent_fields_lpt(h->p)))) {
-    // the line-per-thread kernel (p >= 4) takes them on deformed meshes (4 more loads per
-    // point against the 6 T_lin sweeps) where that measured faster
+    // the line kernel (p >= 4) takes them on deformed meshes (4 more loads per point against the
+    // sweeps of T_lin) where that measured faster
     TRY(ensure_lineark(h));
     a.cf = h->tk;
     law = 7;
