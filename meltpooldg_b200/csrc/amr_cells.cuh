@@ -20,7 +20,7 @@ struct AmrCellArgs {
   // [cell][i][k][j]: a thread's column of n^2 entries is contiguous
   const int *__restrict__ idx;
   const uint16_t *__restrict__ code;
-  const double *__restrict__ src;
+  const double *src;  // (plain loads: a dependent launch's predecessor writes it, launch.cuh)
   const double *__restrict__ Tl;
   // the linearisation point's values and reference gradients at the q-points, [cell][4][n^3]
   const double *__restrict__ tf;
@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(32 * kV2Warps, 4)
 #pragma unroll
     for (int k = 0; k < n; ++k)
 #pragma unroll
-      for (int j = 0; j < n; ++j) Q[k][j] = __ldg(a.src + amr_dof(e[k][j]));
+      for (int j = 0; j < n; ++j) Q[k][j] = a.src[amr_dof(e[k][j])];
 #pragma unroll
     for (int k = 0; k < n; ++k)
 #pragma unroll
@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(32 * kV2Warps, 4)
 #pragma unroll
       for (int k = 0; k < n; ++k)
 #pragma unroll
-        for (int j = 0; j < n; ++j) u[k][j] = __ldg(a.src + amr_dof(e[k][j]));
+        for (int j = 0; j < n; ++j) u[k][j] = a.src[amr_dof(e[k][j])];
 #pragma unroll
       for (int k = 0; k < n; ++k)
 #pragma unroll
@@ -394,9 +394,8 @@ __global__ void k_amr_cg_init(int64_t n, const double *__restrict__ b,
 }
 
 // r -= alpha Ap with the sums r.r and r.D r; the last block tests the convergence
-__global__ void k_amr_cg_update(int64_t n, const double *__restrict__ D,
-                                const double *__restrict__ Ap, double *r, AmrCg *cg,
-                                double *partials, unsigned *counter)
+__global__ void k_amr_cg_update(int64_t n, const double *__restrict__ D, const double *Ap,
+                                double *r, AmrCg *cg, double *partials, unsigned *counter)
 {
   dependents_may_start();
   wait_for_predecessor();
@@ -430,9 +429,8 @@ __global__ void k_amr_cg_update(int64_t n, const double *__restrict__ D,
 
 // x += alpha p, p = D r + beta p, Ap = 0: x is updated where p is read anyway (the iteration that
 // ends the solve leaves it to k_amr_cg_last)
-__global__ void k_amr_cg_direction(int64_t n, const double *__restrict__ D,
-                                   const double *__restrict__ r, double *x, double *p, double *Ap,
-                                   const AmrCg *cg)
+__global__ void k_amr_cg_direction(int64_t n, const double *__restrict__ D, const double *r,
+                                   double *x, double *p, double *Ap, const AmrCg *cg)
 {
   dependents_may_start();
   wait_for_predecessor();
@@ -440,9 +438,9 @@ __global__ void k_amr_cg_direction(int64_t n, const double *__restrict__ D,
   const double alpha = cg->alpha, beta = cg->beta;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
-    const double pi = p[i];
-    x[i] += alpha * pi;
-    p[i] = D[i] * r[i] + beta * pi;
+    const double pi = p[i], xi = x[i], ri = r[i];  // (loaded before the stores)
+    x[i] = xi + alpha * pi;
+    p[i] = D[i] * ri + beta * pi;
     Ap[i] = 0.0;
   }
 }

@@ -39,6 +39,8 @@ template <int LAW> __host__ __device__ constexpr int v2_ncoef()
   return (LAW == 1) ? 4 : (LAW == 2 ? 5 : (LAW == 8 ? 1 : 0));
 }
 constexpr int kV2Warps = 2;  // warps per CTA
+// the instances that are launched as dependents (the FP64 iteration's)
+template <typename T> __host__ __device__ constexpr bool v2_dependent() { return sizeof(T) == 8; }
 // LAW 7's fields per point on register planes: k1 T_lin and k1 dT_lin/dzeta. (The line kernel reads
 // four, {k(T_lin), k1 grad_ref T_lin}.) Storing all four took 1.35 ms per application on 128^3 cells
 // of FE_Q(3), 5.6 GB; these two and the derivatives along the plane 1.25 ms, 3.4 GB (p = 2 0.59 ->
@@ -260,16 +262,23 @@ struct ColumnMask {
   __device__ __forceinline__ bool any() const { return col || ylo || yhi || zlo || zhi; }
 };
 
-// gather a cell's x-column at base (X-layout Q[k][j]); rs, ps: strides of a row and of a plane
-template <int n, typename T>
-__device__ __forceinline__ void gather_column(const T *__restrict__ g, int64_t base, int64_t rs,
-                                              int64_t ps, T (&Q)[n][n], bool active)
+// gather a cell's x-column at base (X-layout Q[k][j]); rs, ps: strides of a row and of a plane.
+// LIVE: plain loads, of a vector that the predecessor of a dependent launch writes (launch.cuh)
+template <int n, bool LIVE = false, typename T>
+__device__ __forceinline__ void gather_column(const T *g, int64_t base, int64_t rs, int64_t ps,
+                                              T (&Q)[n][n], bool active)
 {
   const T *p = g + base;
 #pragma unroll
   for (int k = 0; k < n; ++k)
 #pragma unroll
-    for (int j = 0; j < n; ++j) Q[k][j] = active ? __ldg(p + (rs * j + ps * k)) : T(0);
+    for (int j = 0; j < n; ++j) {
+      const T *q = p + (rs * j + ps * k);
+      if constexpr (LIVE)
+        Q[k][j] = active ? *q : T(0);
+      else
+        Q[k][j] = active ? __ldg(q) : T(0);
+    }
 }
 template <int n, typename T>
 __device__ __forceinline__ void mask_column(const ColumnMask &cm, T (&Q)[n][n])
@@ -363,6 +372,7 @@ __global__ void __launch_bounds__(32 * kV2Warps, (v2_min_blocks<n, T, GEO, LAW>(
   // T_lin (k is affine in T, so this is the conductivity field of LAW 3 without storing it)
   constexpr bool TDEP = LAW == 1 || LAW == 2;
   constexpr bool TLIN = TDEP || LAW == 8;
+  constexpr bool LIVE = v2_dependent<T>();  // the operand is read by plain loads
   dependents_may_start();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -406,7 +416,7 @@ __global__ void __launch_bounds__(32 * kV2Warps, (v2_min_blocks<n, T, GEO, LAW>(
       gather_column<n>(a.src, 4 * cx + t + crs * (J0 + (int64_t)d.nd[1] * K0), crs,
                        crs * d.nd[1], Q, active);
     } else {
-      gather_column<n>(a.src, base, rs, ps, Q, active);
+      gather_column<n, LIVE>(a.src, base, rs, ps, Q, active);
     }
     T Qt[n][n];
     if (TLIN) gather_column<n>(a.Tl, base, rs, ps, Qt, active);
@@ -667,13 +677,13 @@ __global__ void __launch_bounds__(32 * kV2Warps, (v2_min_blocks<n, T, GEO, LAW>(
 
     // ---- optional src.dst partial and the scatter (constrained rows skipped)
     if (!ROWS && a.fin != FIN_NONE && active) {
-      const T *in = a.src + base;
+      T u[n][n];
+      gather_column<n, LIVE>(a.src, base, rs, ps, u, true);
 #pragma unroll
       for (int k = 0; k < n; ++k)
 #pragma unroll
         for (int j = 0; j < n; ++j) {
-          const T u = __ldg(in + (rs * j + ps * k));
-          dot += cm.template at<n>(j, k) ? 0.0 : (double)u * (double)Q[k][j];
+          dot += cm.template at<n>(j, k) ? 0.0 : (double)u[k][j] * (double)Q[k][j];
         }
     }
     bool mine = active;

@@ -116,7 +116,9 @@ struct DegreeOps {
     const int64_t ng = (a.n_cells + v2_cells_per_warp<n>() - 1) / v2_cells_per_warp<n>();
     const int g2 = persistent_grid(k2, 32 * kV2Warps, smem2, (ng + kV2Warps - 1) / kV2Warps, sm,
                                    &cache2);
-    if (a.dependent) return launch_dependent(k2, g2, 32 * kV2Warps, smem2, s, a);
+    if constexpr (v2_dependent<T>()) {
+      if (a.dependent) return launch_dependent(k2, g2, 32 * kV2Warps, smem2, s, a);
+    }
     k2<<<g2, 32 * kV2Warps, smem2, s>>>(a);
     return cudaGetLastError();
   }

@@ -4,6 +4,12 @@
 // predecessor has completed and its writes are visible. Every such kernel waits before its first
 // access to data that another kernel writes, also on the way to an early return. Outside such a
 // launch both calls do nothing.
+//
+// Such a kernel reads the vectors that the iteration writes by plain loads, through pointers
+// without __restrict__. It is resident while its predecessors still write them, and a non-coherent
+// load (__ldg, or what the compiler makes of const __restrict__) is defined only for data that no
+// one writes while the kernel lives; it may also be moved above wait_for_predecessor. What stays
+// fixed during the solve (the diagonal, coefficients, geometry, indices) is read either way.
 #pragma once
 
 #include <cuda_runtime.h>

@@ -652,9 +652,9 @@ __device__ __forceinline__ void finish_iteration(SolverState *st, double rr)
 }
 
 // x += alpha p ; r -= alpha Ap ; rz = r.D r ; rr = r.r ; beta = rz / rz_old
-__global__ void k_cg_update_xr(int64_t N, double *x, double *r, const double *__restrict__ p,
-                               const double *__restrict__ Ap, const double *__restrict__ D,
-                               SolverState *st, double *partials, unsigned *counter)
+__global__ void k_cg_update_xr(int64_t N, double *x, double *r, const double *p, const double *Ap,
+                               const double *__restrict__ D, SolverState *st, double *partials,
+                               unsigned *counter)
 {
   dependents_may_start();
   wait_for_predecessor();
@@ -663,8 +663,9 @@ __global__ void k_cg_update_xr(int64_t N, double *x, double *r, const double *__
   double v[2] = {0.0, 0.0};
   GRID_STRIDE(i, N)
   {
-    x[i] += alpha * p[i];
-    const double ri = r[i] - alpha * Ap[i];
+    const double xi = x[i], pi = p[i], ro = r[i], Api = Ap[i];  // (loaded before the stores)
+    x[i] = xi + alpha * pi;
+    const double ri = ro - alpha * Api;
     r[i] = ri;
     const double zi = D ? D[i] * ri : ri;
     v[0] += ri * zi;
@@ -680,7 +681,7 @@ __global__ void k_cg_update_xr(int64_t N, double *x, double *r, const double *__
 }
 
 // p = D r + beta p ; Ap = 0
-__global__ void k_cg_update_p(int64_t N, const double *__restrict__ r, double *p, double *Ap,
+__global__ void k_cg_update_p(int64_t N, const double *r, double *p, double *Ap,
                               const double *__restrict__ D, const SolverState *st)
 {
   dependents_may_start();
