@@ -20,7 +20,7 @@ struct AmrCellArgs {
   // [cell][i][k][j]: a thread's column of n^2 entries is contiguous
   const int *__restrict__ idx;
   const uint16_t *__restrict__ code;
-  const double *src;  // (plain loads: a dependent launch's predecessor writes it, launch.cuh)
+  const double *src;  // (coherent loads: a dependent launch's predecessor writes it)
   const double *__restrict__ Tl;
   // the linearisation point's values and reference gradients at the q-points, [cell][4][n^3]
   const double *__restrict__ tf;

@@ -82,7 +82,7 @@ struct CellArgs {
   MeshDims d;
   GeoParams<T> g;
   MatParams<T> m;
-  const T *src;  // (plain loads: a dependent launch's predecessor writes it, launch.cuh)
+  const T *src;  // (coherent loads: a dependent launch's predecessor writes it)
   T *dst;
   const T *__restrict__ Tl;
   const T *__restrict__ To;

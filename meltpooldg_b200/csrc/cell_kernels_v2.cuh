@@ -262,23 +262,27 @@ struct ColumnMask {
   __device__ __forceinline__ bool any() const { return col || ylo || yhi || zlo || zhi; }
 };
 
-// gather a cell's x-column at base (X-layout Q[k][j]); rs, ps: strides of a row and of a plane.
-// LIVE: plain loads, of a vector that the predecessor of a dependent launch writes (launch.cuh)
-template <int n, bool LIVE = false, typename T>
-__device__ __forceinline__ void gather_column(const T *g, int64_t base, int64_t rs, int64_t ps,
-                                              T (&Q)[n][n], bool active)
+// gather a cell's x-column at base (X-layout Q[k][j]); rs, ps: strides of a row and of a plane
+template <int n, typename T>
+__device__ __forceinline__ void gather_column(const T *__restrict__ g, int64_t base, int64_t rs,
+                                              int64_t ps, T (&Q)[n][n], bool active)
 {
   const T *p = g + base;
 #pragma unroll
   for (int k = 0; k < n; ++k)
 #pragma unroll
-    for (int j = 0; j < n; ++j) {
-      const T *q = p + (rs * j + ps * k);
-      if constexpr (LIVE)
-        Q[k][j] = active ? *q : T(0);
-      else
-        Q[k][j] = active ? __ldg(q) : T(0);
-    }
+    for (int j = 0; j < n; ++j) Q[k][j] = active ? __ldg(p + (rs * j + ps * k)) : T(0);
+}
+// the same of a vector that the predecessor of a dependent launch writes
+template <int n>
+__device__ __forceinline__ void gather_live(const double *g, int64_t base, int64_t rs, int64_t ps,
+                                            double (&Q)[n][n], bool active)
+{
+  const double *p = g + base;
+#pragma unroll
+  for (int k = 0; k < n; ++k)
+#pragma unroll
+    for (int j = 0; j < n; ++j) Q[k][j] = active ? load_live(p + (rs * j + ps * k)) : 0.0;
 }
 template <int n, typename T>
 __device__ __forceinline__ void mask_column(const ColumnMask &cm, T (&Q)[n][n])
@@ -372,7 +376,6 @@ __global__ void __launch_bounds__(32 * kV2Warps, (v2_min_blocks<n, T, GEO, LAW>(
   // T_lin (k is affine in T, so this is the conductivity field of LAW 3 without storing it)
   constexpr bool TDEP = LAW == 1 || LAW == 2;
   constexpr bool TLIN = TDEP || LAW == 8;
-  constexpr bool LIVE = v2_dependent<T>();  // the operand is read by plain loads
   dependents_may_start();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -415,8 +418,10 @@ __global__ void __launch_bounds__(32 * kV2Warps, (v2_min_blocks<n, T, GEO, LAW>(
       const int64_t crs = 4 * (int64_t)d.m[0];
       gather_column<n>(a.src, 4 * cx + t + crs * (J0 + (int64_t)d.nd[1] * K0), crs,
                        crs * d.nd[1], Q, active);
+    } else if constexpr (v2_dependent<T>()) {
+      gather_live<n>(a.src, base, rs, ps, Q, active);
     } else {
-      gather_column<n, LIVE>(a.src, base, rs, ps, Q, active);
+      gather_column<n>(a.src, base, rs, ps, Q, active);
     }
     T Qt[n][n];
     if (TLIN) gather_column<n>(a.Tl, base, rs, ps, Qt, active);
@@ -678,7 +683,10 @@ __global__ void __launch_bounds__(32 * kV2Warps, (v2_min_blocks<n, T, GEO, LAW>(
     // ---- optional src.dst partial and the scatter (constrained rows skipped)
     if (!ROWS && a.fin != FIN_NONE && active) {
       T u[n][n];
-      gather_column<n, LIVE>(a.src, base, rs, ps, u, true);
+      if constexpr (v2_dependent<T>())
+        gather_live<n>(a.src, base, rs, ps, u, true);
+      else
+        gather_column<n>(a.src, base, rs, ps, u, true);
 #pragma unroll
       for (int k = 0; k < n; ++k)
 #pragma unroll
