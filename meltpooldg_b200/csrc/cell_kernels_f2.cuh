@@ -36,10 +36,6 @@ __device__ __forceinline__ F2 operator-(F2 a, F2 b)
 __device__ __forceinline__ F2 operator*(F2 a, F2 b) { return F2(__fmul2_rn(a.v, b.v)); }
 __device__ __forceinline__ F2 fma(F2 a, F2 b, F2 c) { return F2(__ffma2_rn(a.v, b.v, c.v)); }
 __device__ __forceinline__ F2 operator-(F2 a) { return F2(-a.v.x, -a.v.y); }
-__device__ __forceinline__ F2 minus_twice(F2 a, F2 b)
-{
-  return F2(__ffma2_rn(b.v, make_float2(-2.f, -2.f), a.v));
-}
 template <> __device__ __forceinline__ F2 ctab<F2>(int i) { return F2(c_tab_f2[i]); }
 
 // nodal-grid offset of plane K = p cz + t of a cell, and its corner indices
