@@ -12,36 +12,36 @@ namespace mpdg {
 // entry i of the matrices' table (fill_even_odd); each arithmetic type defines its own
 template <typename T> __device__ __forceinline__ T ctab(int i);
 
-// a - 2 b (one operation)
-__device__ __forceinline__ float minus_twice(float a, float b) { return fmaf(-2.f, b, a); }
-__device__ __forceinline__ double minus_twice(double a, double b) { return fma(-2.0, b, a); }
-
-// y = A x (or y += A x) for the n x n matrix of `kind`, centro-(anti)symmetric. Even-odd split:
-// with E and O the even and odd parts of an output row, y_q accumulates O onto E, all in fused
-// operations. The mirrored output E - O (or O - E) is y_q - 2 E or its negative in FP64, one
-// operation: 14 instead of the 16 operations a row of E + O and E - O at n = 4, 19 instead of 24
-// at n = 5; the plain product is shorter where there is too little to fold, at n = 2 and for
-// y += A x up to n = 4. FP32 keeps the roundings of the separate sums: the mirrored output
-// accumulates -O onto E, and y += A x adds the finished row (y_q - 2 E and accumulation onto y
-// measured 6-12 % more error in the operator).
+// y = A x (or y += A x, which adds the finished row) for the n x n matrix of `kind`,
+// centro-(anti)symmetric. Even-odd split: with E and O the even and odd parts of an output row, the
+// output is E + O and its mirror image E - O (or O - E), h = n / 2 pairs a row.
+//
+// The forms are the shortest whose error is not above that of separately summed parts. Values that
+// vary smoothly over a cell have |E| >> |O|, so it counts how often a sum of E's size is rounded:
+// h + 1 times with separate parts (2 h + 2 operations a pair at even n).
+//   n = 2: the plain product; for the derivatives, where it would round values that cancel, and at
+//     n = 3, O is one product fused onto E.
+//   n = 4, 6 in FP64: E accumulates onto O and the mirror image takes 2 O off again, 2 h + 1
+//     operations, rounded h and h + 1 times (the operator's error 0.91-1.05 of separate parts').
+//   Else separate parts. O accumulated onto E rounds 2 h times at E's size: FP32 in as many
+//     operations at n = 4, 5 and more at 6, 7, with 1.10-1.17 (n = 4), 1.04-1.09 (5), 1.14-1.29 (6, 7)
+//     times the error; FP64 with twice E taken off for the mirror image 1.02-1.19 times.
+// (Emulated operator on sine products, a Gaussian of radius 0.05 and a temperature field; on random
+// operands, where E and O are alike, all forms are within 8 %.) On a B200 the FP64 forms take 1.33 ms
+// for the k(T) tangent on 128^3 cells of FE_Q(3) (with twice E 1.41), 375 us for FE_Q(5) on 53 x 49 x
+// 51 (416), 226 us for FE_Q(6) on 33^3 (218), 158 us for FE_Q(1) on 150^3 (155).
 template <int n, int kind, bool add, typename T>
 __device__ __forceinline__ void contract_row(const T (&x)[n], T (&y)[n])
 {
   constexpr int h = n / 2;
   constexpr int off = tab_off(n, kind);
-  constexpr bool even = kind_sym(kind) > 0, fp64 = std::is_same<T, double>::value;
-  if constexpr (n == 2 || (fp64 && add && n <= 4)) {
+  constexpr bool even = kind_sym(kind) > 0;
+  if constexpr (n == 2 && even) {
     constexpr int full = off + tab_full(n);
-    constexpr bool onto = add && fp64;
-    T r[n];
-#pragma unroll
-    for (int q = 0; q < n; ++q) {
-      r[q] = onto ? fma(ctab<T>(full + q * n), x[0], y[q]) : ctab<T>(full + q * n) * x[0];
-#pragma unroll
-      for (int l = 1; l < n; ++l) r[q] = fma(ctab<T>(full + q * n + l), x[l], r[q]);
-    }
-#pragma unroll
-    for (int q = 0; q < n; ++q) y[q] = add && !onto ? y[q] + r[q] : r[q];
+    const T y0 = fma(ctab<T>(full + 1), x[1], ctab<T>(full) * x[0]);
+    const T y1 = fma(ctab<T>(full + 3), x[1], ctab<T>(full + 2) * x[0]);
+    y[0] = add ? y[0] + y0 : y0;
+    y[1] = add ? y[1] + y1 : y1;
   } else {
     T e[h], o[h];
     const T mid = x[h];
@@ -50,26 +50,33 @@ __device__ __forceinline__ void contract_row(const T (&x)[n], T (&y)[n])
       e[l] = x[l] + x[n - 1 - l];
       o[l] = x[l] - x[n - 1 - l];
     }
+    constexpr bool onto_odd = std::is_same<T, double>::value && n % 2 == 0;
 #pragma unroll
     for (int q = 0; q < h; ++q) {
-      T E = (n & 1) ? ctab<T>(off + 2 * n * h + q) * mid : ctab<T>(off + q * h) * e[0];
+      auto ae = [&](int l) { return ctab<T>(off + q * h + l); };
+      auto ao = [&](int l) { return ctab<T>(off + n * h + q * h + l); };
+      T O = ao(0) * o[0], E, y0, y1;
 #pragma unroll
-      for (int l = (n & 1) ? 0 : 1; l < h; ++l) E = fma(ctab<T>(off + q * h + l), e[l], E);
-      T y0 = E, y1 = E;
+      for (int l = 1; l < h; ++l) O = fma(ao(l), o[l], O);
+      if constexpr (onto_odd) {
+        y0 = O;
 #pragma unroll
-      for (int l = 0; l < h; ++l) y0 = fma(ctab<T>(off + n * h + q * h + l), o[l], y0);
-      // the mirrored output, E - O
-      if constexpr (h > 1 && fp64) {
-        y1 = -minus_twice(y0, E);
+        for (int l = 0; l < h; ++l) y0 = fma(ae(l), e[l], y0);
+        y1 = even ? fma(T(-2), O, y0) : fma(T(2), O, -y0);
       } else {
+        E = (n & 1) ? ctab<T>(off + 2 * n * h + q) * mid : ae(0) * e[0];
 #pragma unroll
-        for (int l = 0; l < h; ++l) y1 = fma(-ctab<T>(off + n * h + q * h + l), o[l], y1);
+        for (int l = (n & 1) ? 0 : 1; l < h; ++l) E = fma(ae(l), e[l], E);
+        if constexpr (h == 1) {
+          y0 = fma(ao(0), o[0], E);
+          y1 = even ? fma(-ao(0), o[0], E) : fma(ao(0), o[0], -E);
+        } else {
+          y0 = E + O;
+          y1 = even ? E - O : O - E;
+        }
       }
       y[q] = add ? y[q] + y0 : y0;
-      if (even)
-        y[n - 1 - q] = add ? y[n - 1 - q] + y1 : y1;
-      else
-        y[n - 1 - q] = add ? y[n - 1 - q] - y1 : -y1;
+      y[n - 1 - q] = add ? y[n - 1 - q] + y1 : y1;
     }
     if constexpr (n & 1) {  // the middle row has only its even (or odd) part
       T c = even ? ctab<T>(off + 2 * n * h + h) * mid : ctab<T>(off + n * h + h * h) * o[0];
