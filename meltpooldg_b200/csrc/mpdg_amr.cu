@@ -29,13 +29,13 @@
 #include <stdexcept>
 #include <string>
 #include <unordered_map>
-#include <map>
 #include <mutex>
 #include <vector>
 
 #include "../../include/mpdg_heat.h"
 #include "amr_cells.cuh"
 #include "fe_tables.hpp"
+#include "resident.hpp"
 
 int mpdg_internal_fail(int code, const char *msg);
 
@@ -886,36 +886,17 @@ AmrArgs make_args(const mpdg_amr *h, const double *T_lin)
 
 enum { CELL_DIAG = 1, CELL_RHS = 2 };
 
-// a persistent grid of as many CTAs as the SMs hold at once, for n_jobs CTAs' worth of work
+// a persistent grid: the CTAs that the device holds at once, at most n_jobs
 constexpr int kAmrMaxBlocks = 148 * 32;
-template <typename K> int resident_grid(K kernel, int threads, int64_t n_jobs, size_t smem = 0)
+template <typename K>
+cudaError_t resident_grid(ResidentBlocks &resident, K kernel, int threads, size_t smem,
+                          int64_t n_jobs, int *grid)
 {
-  static std::mutex mu;
-  static std::map<const void *, int> per_sm_of;  // per kernel
-  static int sms = 0;
-  int per_sm = 0;
-  {
-    std::lock_guard<std::mutex> lock(mu);
-    if (sms == 0) {
-      int dev = 0;
-      cudaGetDevice(&dev);
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    }
-    auto it = per_sm_of.find(reinterpret_cast<const void *>(kernel));
-    if (it == per_sm_of.end()) {
-      if (smem > 48 * 1024)
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) !=
-            cudaSuccess ||
-          per_sm < 1)
-        per_sm = smem ? 1 : 16;
-      per_sm_of[reinterpret_cast<const void *>(kernel)] = per_sm;
-    } else {
-      per_sm = it->second;
-    }
-  }
-  return (int)std::max<int64_t>(
-    1, std::min<int64_t>(std::min<int64_t>(n_jobs, kAmrMaxBlocks), (int64_t)per_sm * sms));
+  int blocks = 0;
+  const cudaError_t e = resident.get(kernel, threads, smem, &blocks);
+  *grid = (int)std::max<int64_t>(
+    1, std::min<int64_t>(std::min<int64_t>(n_jobs, kAmrMaxBlocks), blocks));
+  return e;
 }
 
 // arguments of the register-resident kernels
@@ -940,59 +921,69 @@ AmrCellArgs make_cell_args(const mpdg_amr *h, const double *T_lin)
 }
 
 template <int n, bool TANGENT, bool EVAL>
-void launch_apply(const AmrCellArgs &a, AmrCg *cg, double *partials, unsigned *counter)
+cudaError_t launch_apply(const AmrCellArgs &a, AmrCg *cg, double *partials, unsigned *counter)
 {
+  static ResidentBlocks resident;
   auto k = k_amr_apply<n, TANGENT, EVAL>;
   constexpr size_t smem = amr_smem<n, EVAL>();
-  constexpr int cells = kV2Warps * v2_cells_per_warp<n>();
-  const int g = resident_grid(k, 32 * kV2Warps, (a.n_cells + cells - 1) / cells, smem);
-  if (cg)  // (an error is read by the caller's cudaGetLastError)
-    launch_dependent(k, g, 32 * kV2Warps, smem, (cudaStream_t)0, a, cg, partials, counter);
-  else
-    k<<<g, 32 * kV2Warps, smem>>>(a, cg, partials, counter);
+  constexpr int cells = kV2Warps * v2_cells_per_warp<n>(), threads = 32 * kV2Warps;
+  int g = 0;
+  const cudaError_t e =
+    resident_grid(resident, k, threads, smem, (a.n_cells + cells - 1) / cells, &g);
+  if (e != cudaSuccess) return e;
+  if (cg) return launch_dependent(k, g, threads, smem, (cudaStream_t)0, a, cg, partials, counter);
+  k<<<g, threads, smem>>>(a, cg, partials, counter);
+  return cudaGetLastError();
 }
-template <int n> void launch_tfields(const AmrCellArgs &a, double *tf)
+template <int n> cudaError_t launch_tfields(const AmrCellArgs &a, double *tf)
 {
+  static ResidentBlocks resident;
   auto k = k_amr_tfields<n>;
   constexpr size_t smem = amr_smem<n, false>();
-  constexpr int cells = kV2Warps * v2_cells_per_warp<n>();
-  const int g = resident_grid(k, 32 * kV2Warps, (a.n_cells + cells - 1) / cells, smem);
-  k<<<g, 32 * kV2Warps, smem>>>(a, tf);
+  constexpr int cells = kV2Warps * v2_cells_per_warp<n>(), threads = 32 * kV2Warps;
+  int g = 0;
+  const cudaError_t e =
+    resident_grid(resident, k, threads, smem, (a.n_cells + cells - 1) / cells, &g);
+  if (e != cudaSuccess) return e;
+  k<<<g, threads, smem>>>(a, tf);
+  return cudaGetLastError();
 }
 template <int n>
-void launch_apply_n(const AmrCellArgs &a, bool tangent, AmrCg *cg, double *partials,
-                    unsigned *counter)
+cudaError_t launch_apply_n(const AmrCellArgs &a, bool tangent, AmrCg *cg, double *partials,
+                           unsigned *counter)
 {
-  if (!tangent)
-    launch_apply<n, false, false>(a, cg, partials, counter);
-  else if (a.tf)
-    launch_apply<n, true, false>(a, cg, partials, counter);
-  else
-    launch_apply<n, true, true>(a, cg, partials, counter);
+  if (!tangent) return launch_apply<n, false, false>(a, cg, partials, counter);
+  if (a.tf) return launch_apply<n, true, false>(a, cg, partials, counter);
+  return launch_apply<n, true, true>(a, cg, partials, counter);
 }
 
 template <int n>
-void launch_n(int kind, const AmrArgs &a)
+cudaError_t launch_n(int kind, const AmrArgs &a)
 {
+  static ResidentBlocks resident[2];
   constexpr int n3 = n * n * n;
-  if (kind == CELL_DIAG) {
-    k_amr_diag<n><<<resident_grid(k_amr_diag<n>, n3, a.n_cells), n3>>>(a);
-  } else {
-    k_amr_rhs<n><<<resident_grid(k_amr_rhs<n>, n3, a.n_cells), n3>>>(a);
-  }
+  auto k = kind == CELL_DIAG ? k_amr_diag<n> : k_amr_rhs<n>;
+  int g = 0;
+  const cudaError_t e = resident_grid(resident[kind == CELL_DIAG], k, n3, 0, a.n_cells, &g);
+  if (e != cudaSuccess) return e;
+  k<<<g, n3>>>(a);
+  return cudaGetLastError();
+}
+
+int cuda_status(cudaError_t e)
+{
+  return e == cudaSuccess ? MPDG_OK : fail(MPDG_ERR_CUDA, cudaGetErrorString(e));
 }
 
 int launch_cells(const mpdg_amr *h, int kind, const AmrArgs &a)
 {
   switch (h->n) {
-    case 2: launch_n<2>(kind, a); break;
-    case 3: launch_n<3>(kind, a); break;
-    case 4: launch_n<4>(kind, a); break;
-    case 5: launch_n<5>(kind, a); break;
+    case 2: return cuda_status(launch_n<2>(kind, a));
+    case 3: return cuda_status(launch_n<3>(kind, a));
+    case 4: return cuda_status(launch_n<4>(kind, a));
+    case 5: return cuda_status(launch_n<5>(kind, a));
     default: return fail(MPDG_ERR_INVALID_ARGUMENT, "degree");
   }
-  const cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? MPDG_OK : fail(MPDG_ERR_CUDA, cudaGetErrorString(e));
 }
 
 int ready(const mpdg_amr *h)
@@ -1030,14 +1021,12 @@ int tfields_impl(mpdg_amr *h, const double *T_lin)
   }
   const AmrCellArgs a = make_cell_args(h, T_lin);
   switch (h->n) {
-    case 2: launch_tfields<2>(a, h->tf); break;
-    case 3: launch_tfields<3>(a, h->tf); break;
-    case 4: launch_tfields<4>(a, h->tf); break;
-    case 5: launch_tfields<5>(a, h->tf); break;
+    case 2: return cuda_status(launch_tfields<2>(a, h->tf));
+    case 3: return cuda_status(launch_tfields<3>(a, h->tf));
+    case 4: return cuda_status(launch_tfields<4>(a, h->tf));
+    case 5: return cuda_status(launch_tfields<5>(a, h->tf));
     default: return fail(MPDG_ERR_INVALID_ARGUMENT, "degree");
   }
-  const cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? MPDG_OK : fail(MPDG_ERR_CUDA, cudaGetErrorString(e));
 }
 
 bool is_tangent(const mpdg_amr *h) { return h->mat.law == MPDG_LAW_LINEAR_K && h->mat.k1 != 0.0; }
@@ -1047,14 +1036,12 @@ int apply_cells(const mpdg_amr *h, const AmrCellArgs &a, AmrCg *cg = nullptr)
 {
   const bool tangent = is_tangent(h);
   switch (h->n) {
-    case 2: launch_apply_n<2>(a, tangent, cg, h->partials, h->counter); break;
-    case 3: launch_apply_n<3>(a, tangent, cg, h->partials, h->counter); break;
-    case 4: launch_apply_n<4>(a, tangent, cg, h->partials, h->counter); break;
-    case 5: launch_apply_n<5>(a, tangent, cg, h->partials, h->counter); break;
+    case 2: return cuda_status(launch_apply_n<2>(a, tangent, cg, h->partials, h->counter));
+    case 3: return cuda_status(launch_apply_n<3>(a, tangent, cg, h->partials, h->counter));
+    case 4: return cuda_status(launch_apply_n<4>(a, tangent, cg, h->partials, h->counter));
+    case 5: return cuda_status(launch_apply_n<5>(a, tangent, cg, h->partials, h->counter));
     default: return fail(MPDG_ERR_INVALID_ARGUMENT, "degree");
   }
-  const cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? MPDG_OK : fail(MPDG_ERR_CUDA, cudaGetErrorString(e));
 }
 
 int vmult_impl(mpdg_amr *h, double *dst, const double *src, const double *T_lin)

@@ -206,3 +206,18 @@ def test_solve_stops_at_the_iteration_limit():
         with pytest.raises(H.ExcNoConvergence):
             op.linear_solve(torch.empty_like(b), b, None, rel_tolerance=1e-15,
                             max_iterations=limit)
+
+
+@pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs two devices")
+def test_operator_on_a_second_device():
+    """The k(T) operator evaluated in the kernel needs more than 48 KB of shared memory at p = 3, 4:
+    the limit is raised on every device of the process."""
+    for p in (3, 4):
+        mesh, out = H.box_mesh(p, (4, 3, 3), **BOX), []
+        for dev in (0, 1):
+            op = AmrHeatOperator(mesh, REFINE, device=dev)
+            op.set_material(H.material(law=L.LAW_LINEAR_K, k=1.0, k1=0.5), 1e-2)
+            x = torch.linspace(0.0, 1.0, op.n_dofs, dtype=torch.float64, device=f"cuda:{dev}")
+            with torch.cuda.device(dev):
+                out.append(op.vmult(torch.empty_like(x), x, x).cpu())
+        assert (out[0] - out[1]).abs().max() <= 1e-13 * out[0].abs().max()
