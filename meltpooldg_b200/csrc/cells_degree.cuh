@@ -10,6 +10,7 @@
 #include "cell_kernels_f2.cuh"
 #include "cell_kernels_tc.cuh"
 #include "degree_table.hpp"
+#include "resident.hpp"
 
 #include <stdlib.h>
 #include <algorithm>
@@ -17,21 +18,19 @@
 
 namespace mpdg {
 
-template <typename K>
-static int persistent_grid(K kernel, int threads, size_t smem, int64_t n_batches, int sm_count,
-                           int *cache)
+// a persistent grid: the CTAs that the device holds at once, at most n_batches
+template <typename... P, typename... A>
+static cudaError_t launch_persistent(ResidentBlocks &resident, void (*kernel)(P...), int threads,
+                                     size_t smem, int64_t n_batches, bool dependent,
+                                     cudaStream_t s, const A &...args)
 {
-  if (*cache <= 0) {
-    if (smem > 48 * 1024)
-      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
-    *cache = per_sm > 0 ? per_sm : 1;
-  }
-  int64_t g = (int64_t)(*cache) * sm_count;
-  if (g > n_batches) g = n_batches;
-  if (g < 1) g = 1;
-  return (int)g;
+  int blocks = 0;
+  const cudaError_t e = resident.get(kernel, threads, smem, &blocks);
+  if (e != cudaSuccess) return e;
+  const int g = (int)std::max<int64_t>(1, std::min<int64_t>(blocks, n_batches));
+  if (dependent) return launch_dependent(kernel, g, threads, smem, s, args...);
+  kernel<<<g, threads, smem, s>>>(args...);
+  return cudaGetLastError();
 }
 
 // FP32 operator on the scalar register-resident kernel (default) or the packed-pair
@@ -52,6 +51,15 @@ template <int n>
 struct DegreeOps {
   static constexpr int CPB = cells_per_block(n);
   static constexpr int THREADS = block_threads(n);
+  static constexpr int PLANE_THREADS = 32 * kV2Warps;  // register-plane kernels
+
+  // CTAs' worth of work of the line kernels, and of the register-plane kernels
+  static int64_t line_batches(int64_t cells) { return (cells + CPB - 1) / CPB; }
+  static int64_t plane_batches(int64_t cells)
+  {
+    const int64_t groups = (cells + v2_cells_per_warp<n>() - 1) / v2_cells_per_warp<n>();
+    return (groups + kV2Warps - 1) / kV2Warps;
+  }
 
   static void upload(const double *tab, const float *tabf, const double *w, const float *wf)
   {
@@ -85,14 +93,11 @@ struct DegreeOps {
   {
     if constexpr (std::is_same<T, float>::value && n <= 4 && (LAW == 0 || LAW == 1 || LAW == 3)) {
       if (fp32_packed()) {
-        static int cachep = 0;
+        static ResidentBlocks cachep;
         auto kp = k_vmult2p<n, GEO, LAW>;
         const size_t smemp = v2_smem<n, F2, LAW>();
-        const int64_t ng = ((a.n_cells + 1) / 2 + v2_cells_per_warp<n>() - 1) / v2_cells_per_warp<n>();
-        const int gp = persistent_grid(kp, 32 * kV2Warps, smemp, (ng + kV2Warps - 1) / kV2Warps,
-                                       sm, &cachep);
-        kp<<<gp, 32 * kV2Warps, smemp, s>>>(a);
-        return cudaGetLastError();
+        return launch_persistent(cachep, kp, PLANE_THREADS, smemp,
+                                 plane_batches((a.n_cells + 1) / 2), false, s, a);
       }
     }
     // at p = 5 only where the cells fill a round of the grid (8 warps per SM): below that the time
@@ -108,29 +113,22 @@ struct DegreeOps {
   template <typename T, int GEO, int LAW>
   static cudaError_t vmult_planes(const CellArgs<T> &a, cudaStream_t s, int sm)
   {
-    static int cache2 = 0;
+    static ResidentBlocks cache2;
     // deformed FP64: the geometry from the cell's vertices (p >= 2) instead of the stored one
     constexpr int G = v2_geometry<n, T, GEO>();
     auto k2 = k_vmult2<n, T, G, LAW>;
     const size_t smem2 = v2_smem<n, T, LAW, G>();
-    const int64_t ng = (a.n_cells + v2_cells_per_warp<n>() - 1) / v2_cells_per_warp<n>();
-    const int g2 = persistent_grid(k2, 32 * kV2Warps, smem2, (ng + kV2Warps - 1) / kV2Warps, sm,
-                                   &cache2);
-    if constexpr (v2_dependent<T>()) {
-      if (a.dependent) return launch_dependent(k2, g2, 32 * kV2Warps, smem2, s, a);
-    }
-    k2<<<g2, 32 * kV2Warps, smem2, s>>>(a);
-    return cudaGetLastError();
+    const bool dependent = v2_dependent<T>() && a.dependent;
+    return launch_persistent(cache2, k2, PLANE_THREADS, smem2, plane_batches(a.n_cells), dependent,
+                             s, a);
   }
   template <typename T, int GEO, int LAW>
   static cudaError_t vmult_lines(const CellArgs<T> &a, cudaStream_t s, int sm)
   {
-    static int cache = 0;
+    static ResidentBlocks cache;
     auto k = k_vmult_lines<n, T, ln_geometry<T, GEO, LAW>(), LAW>;
     constexpr size_t smem = ln_smem<n, T>();
-    const int g = persistent_grid(k, THREADS, smem, (a.n_cells + CPB - 1) / CPB, sm, &cache);
-    k<<<g, THREADS, smem, s>>>(a);
-    return cudaGetLastError();
+    return launch_persistent(cache, k, THREADS, smem, line_batches(a.n_cells), false, s, a);
   }
   template <typename T>
   static cudaError_t vmult(const CellArgs<T> &a, int geo, int law, cudaStream_t s, int sm)
@@ -181,22 +179,17 @@ struct DegreeOps {
   static cudaError_t rhs_t(const CellArgs<double> &a, cudaStream_t s, int sm)
   {
     if constexpr (use_v2<double>() && (LAW == 0 || LAW == 1)) {
-      static int cache2 = 0;
+      static ResidentBlocks cache2;
       auto k2 = k_rhs2<n, GEO, LAW>;
       const size_t smem2 =
         sizeof(double) * kV2Warps * 2 * (v2_cells_per_warp<n>() + 1) * v2_cell_stride<n>();
-      const int64_t ng = (a.n_cells + v2_cells_per_warp<n>() - 1) / v2_cells_per_warp<n>();
-      const int g2 = persistent_grid(k2, 32 * kV2Warps, smem2, (ng + kV2Warps - 1) / kV2Warps, sm,
-                                     &cache2);
-      k2<<<g2, 32 * kV2Warps, smem2, s>>>(a);
-      return cudaGetLastError();
+      return launch_persistent(cache2, k2, PLANE_THREADS, smem2, plane_batches(a.n_cells), false, s,
+                               a);
     }
-    static int cache = 0;
+    static ResidentBlocks cache;
     auto k = k_rhs<n, GEO, LAW>;
     const size_t smem = smem_rhs<n>();
-    const int g = persistent_grid(k, THREADS, smem, (a.n_cells + CPB - 1) / CPB, sm, &cache);
-    k<<<g, THREADS, smem, s>>>(a);
-    return cudaGetLastError();
+    return launch_persistent(cache, k, THREADS, smem, line_batches(a.n_cells), false, s, a);
   }
   static cudaError_t rhs(const CellArgs<double> &a, int geo, int law, cudaStream_t s, int sm)
   {
@@ -216,14 +209,11 @@ struct DegreeOps {
   static cudaError_t diag_t(const CellArgs<double> &a, cudaStream_t s, int sm)
   {
     if constexpr (use_v2<double>() && (LAW == 0 || LAW == 1)) {
-      static int cache2 = 0;
+      static ResidentBlocks cache2;
       auto k2 = k_diag2<n, GEO, LAW>;
       constexpr size_t smem2 = diag2_smem<n, LAW>();
-      const int64_t ng = (a.n_cells + v2_cells_per_warp<n>() - 1) / v2_cells_per_warp<n>();
-      const int g2 = persistent_grid(k2, 32 * kV2Warps, smem2, (ng + kV2Warps - 1) / kV2Warps, sm,
-                                     &cache2);
-      k2<<<g2, 32 * kV2Warps, smem2, s>>>(a);
-      return cudaGetLastError();
+      return launch_persistent(cache2, k2, PLANE_THREADS, smem2, plane_batches(a.n_cells), false, s,
+                               a);
     } else {
       return diag_lines<GEO, LAW>(a, s, sm);
     }
@@ -231,12 +221,10 @@ struct DegreeOps {
   template <int GEO, int LAW>
   static cudaError_t diag_lines(const CellArgs<double> &a, cudaStream_t s, int sm)
   {
-    static int cache = 0;
+    static ResidentBlocks cache;
     auto k = k_diag<n, GEO, LAW>;
     const size_t smem = smem_diag<n>();
-    const int g = persistent_grid(k, THREADS, smem, (a.n_cells + CPB - 1) / CPB, sm, &cache);
-    k<<<g, THREADS, smem, s>>>(a);
-    return cudaGetLastError();
+    return launch_persistent(cache, k, THREADS, smem, line_batches(a.n_cells), false, s, a);
   }
   static cudaError_t diag(const CellArgs<double> &a, int geo, int law, cudaStream_t s, int sm)
   {
@@ -255,12 +243,10 @@ struct DegreeOps {
   template <int GEO>
   static cudaError_t norm_t(const CellArgs<double> &a, cudaStream_t s, int sm)
   {
-    static int cache = 0;
+    static ResidentBlocks cache;
     auto k = k_norm<n, GEO>;
     const size_t smem = smem_norm<n>();
-    const int g = persistent_grid(k, THREADS, smem, (a.n_cells + CPB - 1) / CPB, sm, &cache);
-    k<<<g, THREADS, smem, s>>>(a);
-    return cudaGetLastError();
+    return launch_persistent(cache, k, THREADS, smem, line_batches(a.n_cells), false, s, a);
   }
   static cudaError_t norm(const CellArgs<double> &a, int geo, int, cudaStream_t s, int sm)
   {
@@ -270,24 +256,22 @@ struct DegreeOps {
   template <int LAW>
   static cudaError_t kq_t(const CellArgs<double> &a, float *kq, cudaStream_t s, int sm)
   {
-    static int cache = 0;
+    static ResidentBlocks cache;
     auto k = k_conductivity_q<n, LAW>;
-    const size_t smem = sizeof(double) * kV2Warps * (v2_cells_per_warp<n>() + 1) * v2_cell_stride<n>();
-    const int64_t ng = (a.n_cells + v2_cells_per_warp<n>() - 1) / v2_cells_per_warp<n>();
-    const int g = persistent_grid(k, 32 * kV2Warps, smem, (ng + kV2Warps - 1) / kV2Warps, sm, &cache);
-    k<<<g, 32 * kV2Warps, smem, s>>>(a, kq);
-    return cudaGetLastError();
+    const size_t smem =
+      sizeof(double) * kV2Warps * (v2_cells_per_warp<n>() + 1) * v2_cell_stride<n>();
+    return launch_persistent(cache, k, PLANE_THREADS, smem, plane_batches(a.n_cells), false, s,
+                             a, kq);
   }
   template <int GEO>
   static cudaError_t diag_picard_t(const CellArgs<float> &a, cudaStream_t s, int sm)
   {
-    static int cache = 0;
+    static ResidentBlocks cache;
     auto k = k_diag_picard<n, GEO>;
-    const size_t smem = sizeof(float) * kV2Warps * 2 * (v2_cells_per_warp<n>() + 1) * v2_cell_stride<n>();
-    const int64_t ng = (a.n_cells + v2_cells_per_warp<n>() - 1) / v2_cells_per_warp<n>();
-    const int g = persistent_grid(k, 32 * kV2Warps, smem, (ng + kV2Warps - 1) / kV2Warps, sm, &cache);
-    k<<<g, 32 * kV2Warps, smem, s>>>(a);
-    return cudaGetLastError();
+    const size_t smem =
+      sizeof(float) * kV2Warps * 2 * (v2_cells_per_warp<n>() + 1) * v2_cell_stride<n>();
+    return launch_persistent(cache, k, PLANE_THREADS, smem, plane_batches(a.n_cells), false, s,
+                             a);
   }
   static cudaError_t diag_picard(const CellArgs<float> &a, int geo, cudaStream_t s, int sm)
   {
@@ -296,13 +280,11 @@ struct DegreeOps {
   template <int GEO>
   static cudaError_t vmult_picard_rows_t(const CellArgs<float> &a, cudaStream_t s, int sm)
   {
-    static int cache = 0;
+    static ResidentBlocks cache;
     auto k = k_vmult2<n, float, GEO, 3, true>;
     const size_t smem = v2_smem<n, float, 3>();
-    const int64_t ng = (a.n_cells + v2_cells_per_warp<n>() - 1) / v2_cells_per_warp<n>();
-    const int g = persistent_grid(k, 32 * kV2Warps, smem, (ng + kV2Warps - 1) / kV2Warps, sm, &cache);
-    k<<<g, 32 * kV2Warps, smem, s>>>(a);
-    return cudaGetLastError();
+    return launch_persistent(cache, k, PLANE_THREADS, smem, plane_batches(a.n_cells), false, s,
+                             a);
   }
   static cudaError_t vmult_picard_rows(const CellArgs<float> &a, int geo, cudaStream_t s, int sm)
   {
@@ -317,14 +299,10 @@ struct DegreeOps {
                                      cudaStream_t s, int sm)
   {
     if constexpr (n == 4) {
-      static bool attr = false;
+      static SharedLimit limit;
       auto k = k_vmult_picard_tc<n>;
-      if (!attr) {
-        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)optc::kSmem);
-        if (e != cudaSuccess) return e;
-        attr = true;
-      }
+      const cudaError_t e = limit.raise(k, optc::kSmem);
+      if (e != cudaSuccess) return e;
       const int64_t nb = (int64_t)((a.d.m[0] + optc::kBX - 1) / optc::kBX) *
                          ((a.d.m[1] + optc::kBY - 1) / optc::kBY) *
                          ((a.d.m[2] + optc::kBZ - 1) / optc::kBZ);
@@ -341,12 +319,10 @@ struct DegreeOps {
   template <int GEO>
   static cudaError_t coef_tangent_t(const CellArgs<double> &a, double *out, cudaStream_t s, int sm)
   {
-    static int cache = 0;
+    static ResidentBlocks cache;
     auto k = k_coef_tangent<n, GEO>;
     const size_t smem = smem_coef_tangent<n>();
-    const int g = persistent_grid(k, THREADS, smem, (a.n_cells + CPB - 1) / CPB, sm, &cache);
-    k<<<g, THREADS, smem, s>>>(a, out);
-    return cudaGetLastError();
+    return launch_persistent(cache, k, THREADS, smem, line_batches(a.n_cells), false, s, a, out);
   }
   static cudaError_t coef_tangent(const CellArgs<double> &a, double *out, int geo, cudaStream_t s,
                                   int sm)
@@ -355,32 +331,27 @@ struct DegreeOps {
   }
   static cudaError_t coef_lineark(const CellArgs<double> &a, double *out, cudaStream_t s, int sm)
   {
-    static int cache = 0;
+    static ResidentBlocks cache;
     if constexpr (use_v2<double>()) {
       auto k = k_coef_lineark2<n>;
       constexpr size_t smem =
         sizeof(double) * kV2Warps * 2 * (v2_cells_per_warp<n>() + 1) * v2_cell_stride<n>();
-      const int64_t ng = (a.n_cells + v2_cells_per_warp<n>() - 1) / v2_cells_per_warp<n>();
-      const int g = persistent_grid(k, 32 * kV2Warps, smem, (ng + kV2Warps - 1) / kV2Warps, sm,
-                                    &cache);
-      k<<<g, 32 * kV2Warps, smem, s>>>(a, out);
+      return launch_persistent(cache, k, PLANE_THREADS, smem, plane_batches(a.n_cells), false, s, a,
+                               out);
     } else {
       auto k = k_coef_lineark<n>;
       const size_t smem = smem_coef_lineark<n>();
-      const int g = persistent_grid(k, THREADS, smem, (a.n_cells + CPB - 1) / CPB, sm, &cache);
-      k<<<g, THREADS, smem, s>>>(a, out);
+      return launch_persistent(cache, k, THREADS, smem, line_batches(a.n_cells), false, s, a, out);
     }
-    return cudaGetLastError();
   }
   static cudaError_t field_values(const CellArgs<double> &a, const double *H, const double *vel,
                                   int64_t n_dofs, double *cf, cudaStream_t s, int sm)
   {
-    static int cache = 0;
+    static ResidentBlocks cache;
     auto k = k_field_values<n>;
     const size_t smem = smem_norm<n>();
-    const int g = persistent_grid(k, THREADS, smem, (a.n_cells + CPB - 1) / CPB, sm, &cache);
-    k<<<g, THREADS, smem, s>>>(a, H, vel, n_dofs, cf);
-    return cudaGetLastError();
+    return launch_persistent(cache, k, THREADS, smem, line_batches(a.n_cells), false, s, a, H, vel,
+                             n_dofs, cf);
   }
   static cudaError_t conductivity_q(const CellArgs<double> &a, float *kq, int law, cudaStream_t s,
                                     int sm)

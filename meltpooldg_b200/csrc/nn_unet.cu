@@ -38,6 +38,7 @@
 #include "nn_conv_tc.cuh"
 #include "nn_wgrad.cuh"
 #include "reduce.cuh"
+#include "resident.hpp"
 
 using namespace mpdg;
 
@@ -380,7 +381,8 @@ int wgrad_t(mpdg_unet *u, const nn_wg::Args &args)
   auto k = nn_wg::k_wgrad<CI, CG>;
   nn_wg::Args a = args;
   constexpr size_t smem = nn_wg::smem_bytes<CI, CG>();
-  NNCU(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  static SharedLimit limit;
+  NNCU(limit.raise(k, smem));
   a.ci_groups = (a.ci + CI - 1) / CI;
   const int blocks = a.ci_groups * ((a.co + 4 * CG - 1) / (4 * CG));
   const int64_t tiles = (int64_t)((a.nx + nn_wg::kX - 1) / nn_wg::kX) *
@@ -448,8 +450,7 @@ int tc_launch(mpdg_unet *u, Grid3 g, int ci, int co, const uint4 *wp, const floa
               const __nv_bfloat16 *in, const __nv_bfloat16 *add, TO *out, const Grid3 *up_from)
 {
   auto k = nn_tc::k_conv3d_tc<NPAD, RELU, ADD, TO>;
-  static size_t attr_smem = 0;  // the attribute is kept at the request of the launch, so
-                                // that the occupancy query sees the real footprint
+  static SharedLimit limit;
   nn_tc::ConvArgs a;
   a.nx = g.nx;
   a.ny = g.ny;
@@ -469,10 +470,7 @@ int tc_launch(mpdg_unet *u, Grid3 g, int ci, int co, const uint4 *wp, const floa
   a.out = out;
   a.err = u->tc_err;
   const size_t smem = nn_tc::smem_bytes(a.cg, NPAD, a.taps_per_stage);
-  if (smem != attr_smem) {
-    NNCU(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attr_smem = smem;
-  }
+  NNCU(limit.raise(k, smem));
   // resident CTAs per SM from registers, shared memory, threads and tensor-memory columns
   static int per_sm_regs = 0, smem_sm = 0, smem_rsv = 0, static_smem = 0;
   if (per_sm_regs == 0) {

@@ -87,3 +87,10 @@ def test_limits_are_set_on_every_device(tmp_path):
                     str(tmp_path / "main.cpp"), "-o", str(exe)], check=True, timeout=120)
     r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, r.stdout
+
+
+def test_no_launch_limit_is_kept_per_process():
+    """Every limit is raised through resident.hpp."""
+    for f in sorted(os.listdir(CSRC)):
+        if f != "resident.hpp":
+            assert "cudaFuncSetAttribute" not in open(os.path.join(CSRC, f)).read(), f
