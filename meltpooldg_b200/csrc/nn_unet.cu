@@ -732,15 +732,20 @@ extern "C" int mpdg_unet_create(int nx, int ny, int nz, uint64_t seed, mpdg_unet
     return rc;
   };
   const int64_t n0 = u->g[0].n(), n1 = u->g[1].n(), n2 = u->g[2].n(), n3 = u->g[3].n();
+  const char *e = getenv("MPDG_UNET_TC");
+  u->use_tc = !(e && e[0] == '0');
+  // the upsampled tensors u0, u1, u2 are formed by the CUDA-core forward only
+  const int64_t up = u->use_tc ? 0 : 1;
   struct A { __nv_bfloat16 **p; int64_t n; } acts[] = {
     {&u->x0, 8 * n0}, {&u->a0, 16 * n0}, {&u->e0, 16 * n0}, {&u->p0, 16 * n1}, {&u->a1, 32 * n1},
     {&u->e1, 32 * n1}, {&u->p1, 32 * n2}, {&u->a2, 48 * n2}, {&u->e2, 48 * n2}, {&u->p2, 48 * n3},
-    {&u->a3, 64 * n3}, {&u->e3, 64 * n3}, {&u->u2, 64 * n2}, {&u->s2, 48 * n2}, {&u->d2, 48 * n2},
-    {&u->u1, 48 * n1}, {&u->s1, 32 * n1}, {&u->d1, 32 * n1}, {&u->u0, 32 * n0}, {&u->s0, 16 * n0},
-    {&u->d0, 16 * n0}};
+    {&u->a3, 64 * n3}, {&u->e3, 64 * n3}, {&u->u2, up * 64 * n2}, {&u->s2, 48 * n2},
+    {&u->d2, 48 * n2}, {&u->u1, up * 48 * n1}, {&u->s1, 32 * n1}, {&u->d1, 32 * n1},
+    {&u->u0, up * 32 * n0}, {&u->s0, 16 * n0}, {&u->d0, 16 * n0}};
   int rc;
   for (auto &a : acts)
-    if ((rc = ualloc(u, (void **)a.p, sizeof(__nv_bfloat16) * a.n)) != MPDG_OK) return fail_free(rc);
+    if (a.n > 0 && (rc = ualloc(u, (void **)a.p, sizeof(__nv_bfloat16) * a.n)) != MPDG_OK)
+      return fail_free(rc);
   const int64_t gmax = std::max(std::max(32 * n0, 48 * n1), std::max(64 * n2, 64 * n3));
   float **fb[] = {&u->y, &u->gA, &u->gB, &u->gC};
   const int64_t fsz[] = {n0, gmax, gmax, gmax};
@@ -781,8 +786,6 @@ extern "C" int mpdg_unet_create(int nx, int ny, int nz, uint64_t seed, mpdg_unet
     return fail_free(rc);
   cudaMemset(u->zero_bias, 0, sizeof(float) * 64);
   {
-    const char *e = getenv("MPDG_UNET_TC");
-    u->use_tc = !(e && e[0] == '0');
     const char *eb = getenv("MPDG_UNET_TC_BWD");
     u->use_tc_bwd = !(eb && eb[0] == '0');
     int dev = 0;

@@ -187,3 +187,20 @@ def test_weight_gradients_at_tile_edges_are_exact(dims):
     assert torch.equal(got[13][0].double(), wo.double().view(16, 1, 1, 1, 1) *
                        c.double().view(1, 16, 1, 1, 1) * taps)
     assert torch.equal(got[13][1].double(), wo.double() * gy.double().sum())
+
+
+def test_upsampled_tensors_are_held_by_the_cuda_core_forward_only(monkeypatch):
+    """Device memory of a network: with the CUDA-core forward larger by its three upsampled decoder
+    inputs (64, 48 and 32 BF16 channels, 42 MB at 81^3), up to the allocator's granularity
+    (2 MB for each of them)."""
+    def taken(mode):
+        monkeypatch.setenv("MPDG_UNET_TC", mode)
+        before = torch.cuda.mem_get_info()[0]
+        net = LG.UNet((81, 81, 81), seed=1)
+        held = before - torch.cuda.mem_get_info()[0]
+        del net
+        return held
+    taken("1")  # what the process loads with its first network
+    n0, n1, n2 = 81 ** 3, 41 ** 3, 21 ** 3
+    ups = 2 * (32 * n0 + 48 * n1 + 64 * n2)
+    assert abs(taken("0") - taken("1") - ups) <= 3 * 2 ** 21
