@@ -101,3 +101,63 @@ def test_application_in_a_cuda_graph(degree, cells):
     rz = op.vmult(op.new_vector(), ry)
     assert (y - ry).abs().max() <= 1e-13 * ry.abs().max()
     assert (z - rz).abs().max() <= 1e-12 * rz.abs().max()
+
+
+FIELD_LAWS = {
+    # material, heaviside, velocity: T_old in the tangent; coefficient fields; both with convection
+    "liquid_solid": (dict(law=2, rho=1.0, cp=1.0, k=0.5, rho_s=1.2, cp_s=0.8, k_s=2.5,
+                          T_solidus=0.3, T_liquidus=0.7), False, False),
+    "gas_liquid_velocity": (dict(law=3, rho=2.0, cp=3.0, k=5.0, rho_g=0.5, cp_g=1.5, k_g=0.3),
+                            True, True),
+    "three_phase_velocity": (dict(law=4, rho=1.0, cp=1.0, k=0.5, rho_s=1.2, cp_s=0.8, k_s=2.5,
+                                  T_solidus=0.3, T_liquidus=0.7, rho_g=0.4, cp_g=1.5, k_g=0.2),
+                             True, True),
+}
+
+
+@pytest.mark.parametrize("degree,cells", [(3, (29, 31, 37)), (4, (23, 29, 31)), (5, (13, 17, 19)),
+                                          (6, (11, 13, 17))])
+@pytest.mark.parametrize("perturb", [0.0, 0.2])
+@pytest.mark.parametrize("law", list(FIELD_LAWS))
+def test_field_laws_over_several_rounds(degree, cells, perturb, law):
+    """The laws that use the line kernel's shared arrays more than once a batch (T_old's values) or
+    read per-point fields, where every block takes several batches. FP64: a phase change's branches
+    are taken at the same points."""
+    m, with_h, with_v = FIELD_LAWS[law]
+    mask, dt = 0b010010, 1e-2
+    o = O.Oracle(degree, cells, perturb=perturb, seed=5, dirichlet_mask=mask)
+    o.set_material(O.material(**m), dt)
+    g = H.HeatDiffuseOperator(H.box_mesh(degree, cells, perturb=perturb, seed=5, dirichlet=(1, 4)))
+    g.set_material(H.material(**m))
+    g.reset_time_increment(dt)
+    x = o.support_points()
+    hv = 0.5 + 0.5 * np.tanh((x[:, 0] - 0.45) / 0.1) if with_h else None
+    v = np.stack([np.sin(3 * x[:, 1]), 0.5 + x[:, 2], -x[:, 0] * x[:, 1]]) if with_v else None
+    o.set_fields(hv, v)
+    g.set_fields(*(None if f is None else torch.tensor(f, device="cuda") for f in (hv, v)))
+    rng = np.random.default_rng(degree)
+    src, Tl, To = (rng.uniform(lo, 1.0, o.n_dofs) for lo in (-1.0, 0.0, 0.0))
+    d = {k: torch.tensor(a, device="cuda") for k, a in dict(src=src, Tl=Tl, To=To).items()}
+    g.set_linearization(d["Tl"], d["To"])
+    assert rel(g.vmult(g.new_vector(), d["src"]), o.vmult(src, Tl, To)) <= TOL64
+
+
+@pytest.mark.parametrize("degree", [1, 2, 3])
+@pytest.mark.parametrize("cells", [(1, 1, 1), (33, 1, 2), (2, 17, 3), "long"])
+@pytest.mark.parametrize("perturb", [0.0, 0.2])
+@pytest.mark.parametrize("law", ["constant", "linear_k"])
+def test_inverse_diagonal(degree, cells, perturb, law):
+    """The register-plane diagonal on one cell, on rows one cell wide and over several rounds."""
+    cells = LONG[degree] if cells == "long" else cells
+    m = KT if law == "linear_k" else dict(law=0, rho=1.0, cp=1.0, k=1.0)
+    mask, dt = 0b000001, 1e-3
+    o = O.Oracle(degree, cells, perturb=perturb, seed=5, dirichlet_mask=mask)
+    o.set_material(O.material(**m), dt)
+    g = H.HeatDiffuseOperator(H.box_mesh(degree, cells, perturb=perturb, seed=5, dirichlet=(0,)))
+    g.set_material(H.material(**m))
+    g.reset_time_increment(dt)
+    Tl = np.random.default_rng(degree).uniform(0.0, 1.0, o.n_dofs)
+    Td = torch.tensor(Tl, device="cuda")
+    g.set_linearization(Td, Td)
+    d = g.compute_inverse_diagonal_from_matrixfree(g.new_vector())
+    assert rel(1.0 / d, 1.0 / o.inverse_diagonal(Tl, Tl)) <= TOL64
