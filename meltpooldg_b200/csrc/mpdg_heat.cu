@@ -967,14 +967,15 @@ __global__ void k_inject(Dims3 fd, Dims3 cd, int r, const double *__restrict__ f
 
 // Transfers along one axis of a tensor [outer][axis][inner] (inner fastest). Restriction sweeps z,
 // y, x and the prolongation x, y, z, so the large arrays meet the sweep along z, where a thread's
-// values are one inner index over a run of kRun coarse nodes: lanes read and write contiguous rows
-// and every fine value is touched once. (With x first, each lane gathered 2 r - 1 values r apart
+// values are one inner index over a run of coarse nodes: lanes read and write contiguous rows and
+// every fine value is touched once. (With x first, each lane gathered 2 r - 1 values r apart
 // through index divisions: level 0 at 57 M DoFs, residual restricted and prolonged back, 0.89 ms a
 // V-cycle against 0.42 ms.)
 constexpr int kRun = 8;
 struct TransferArgs {
   int64_t inner, outer;
   int n_fine, n_coarse, r;  // nodes along the axis: n_fine = r (n_coarse - 1) + 1
+  int run;                  // coarse nodes a thread, at most kRun
   float xi[8];              // position of fine node a (0 <= a < r) in its coarse interval
 };
 
@@ -983,12 +984,12 @@ __device__ __forceinline__ bool run_index(const TransferArgs &t, int64_t &i, int
                                           int &V1)
 {
   const unsigned nb = (unsigned)((t.inner + VT - 1) / VT),
-                 runs = (unsigned)((t.n_coarse + kRun - 1) / kRun);
+                 runs = (unsigned)((t.n_coarse + t.run - 1) / t.run);
   const unsigned q = blockIdx.x / nb, ib = blockIdx.x - q * nb;
   o = q / runs;
   i = (int64_t)ib * VT + threadIdx.x;
-  V0 = (int)(q - (unsigned)o * runs) * kRun;
-  V1 = min(V0 + kRun, t.n_coarse);
+  V0 = (int)(q - (unsigned)o * runs) * t.run;
+  V1 = min(V0 + t.run, t.n_coarse);
   return i < t.inner;
 }
 
@@ -2282,10 +2283,16 @@ static TransferArgs transfer_args(const MGLevel &f, const Dims3 &F, const Dims3 
   t.outer = 1;  // and of those after it
   return t;
 }
-// (a level holds < 2^31 nodes, so the blocks fit the grid's first dimension)
-static unsigned run_grid(const TransferArgs &t)
+// The blocks of a sweep along y or z (a level holds < 2^31 nodes, so they fit the grid's first
+// dimension), and the run length: kRun where that leaves two blocks an SM, else half of it until it
+// does: on a small level a run is a chain of loads that nothing else hides (a step on 16^3 cells of
+// FE_Q(3) 1.87 ms with runs of 8 throughout, 1.74 ms).
+static unsigned run_grid(const mpdg_heat *h, TransferArgs &t)
 {
-  return (unsigned)((t.inner + VT - 1) / VT * ((t.n_coarse + kRun - 1) / kRun) * t.outer);
+  const int64_t across = (t.inner + VT - 1) / VT * t.outer;
+  t.run = kRun;
+  while (t.run > 1 && across * ((t.n_coarse + t.run - 1) / t.run) < 2 * h->sm_count) t.run /= 2;
+  return (unsigned)(across * ((t.n_coarse + t.run - 1) / t.run));
 }
 static int mg_restrict(mpdg_heat *h, int l, const float *fine_Ax, const float *fine_b,
                        float *coarse)
@@ -2298,11 +2305,13 @@ static int mg_restrict(mpdg_heat *h, int l, const float *fine_Ax, const float *f
            : t.r == 4 ? k_restrict_run<4>
                       : k_restrict_run<0>;
   t.inner = (int64_t)F.n[0] * F.n[1];
-  k<<<run_grid(t), VT, 0, h->stream>>>(t, fine_Ax, fine_b, h->mg_t1, h->st);
+  unsigned grid = run_grid(h, t);
+  k<<<grid, VT, 0, h->stream>>>(t, fine_Ax, fine_b, h->mg_t1, h->st);
   t = transfer_args(f, F, C, 1);
   t.inner = F.n[0];
   t.outer = C.n[2];
-  k<<<run_grid(t), VT, 0, h->stream>>>(t, h->mg_t1, nullptr, h->mg_t2, h->st);
+  grid = run_grid(h, t);
+  k<<<grid, VT, 0, h->stream>>>(t, h->mg_t1, nullptr, h->mg_t2, h->st);
   t = transfer_args(f, F, C, 0);
   k_restrict_x<<<vgrid(h, C.size()), VT, 0, h->stream>>>((int64_t)C.n[1] * C.n[2], t, h->mg_t2,
                                                          coarse, c.h->dims, h->st);
@@ -2328,8 +2337,8 @@ static int mg_prolong_add(mpdg_heat *h, int l, const float *coarse, float *fine,
             : t.r == 3 ? k_prolong_run<3, false, false>
             : t.r == 4 ? k_prolong_run<4, false, false>
                        : k_prolong_run<0, false, false>;
-  ky<<<run_grid(t), VT, 0, h->stream>>>(t, h->mg_t2, h->mg_t1, f.h->dims, nullptr, h->st,
-                                                CellRows());
+  unsigned grid = run_grid(h, t);
+  ky<<<grid, VT, 0, h->stream>>>(t, h->mg_t2, h->mg_t1, f.h->dims, nullptr, h->st, CellRows());
   t = transfer_args(f, F, C, 2);
   t.inner = (int64_t)F.n[0] * F.n[1];
   auto kz = fine_rows.rows ? k_prolong_run<0, true, true>
@@ -2337,7 +2346,8 @@ static int mg_prolong_add(mpdg_heat *h, int l, const float *coarse, float *fine,
             : t.r == 3     ? k_prolong_run<3, true, false>
             : t.r == 4     ? k_prolong_run<4, true, false>
                            : k_prolong_run<0, true, false>;
-  kz<<<run_grid(t), VT, 0, h->stream>>>(t, h->mg_t1, fine, f.h->dims, zero_fine, h->st, fine_rows);
+  grid = run_grid(h, t);
+  kz<<<grid, VT, 0, h->stream>>>(t, h->mg_t1, fine, f.h->dims, zero_fine, h->st, fine_rows);
   h->launches += 3;
   CU(cudaGetLastError());
   return MPDG_OK;

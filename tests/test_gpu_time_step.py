@@ -520,3 +520,9 @@ def test_multigrid_on_unequal_boxes(degree, cells, perturb):
     H.LinearSolver.solve(op, xp, b, H.LinearSolverData(rel_tolerance=1e-12, abs_tolerance=0.0), jac)
     assert its <= 25
     assert (x - xp).norm().item() <= 1e-8 * xp.norm().item()
+
+
+@pytest.mark.parametrize("cells", [(24, 24, 24), (28, 28, 28), (32, 32, 32)])
+def test_multigrid_run_lengths(cells):
+    """The transfers' runs of 1, 2 and 4 coarse nodes a thread on the finest level (148 SMs)."""
+    test_multigrid_on_unequal_boxes(3, cells, 0.0)
