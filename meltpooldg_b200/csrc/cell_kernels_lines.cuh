@@ -13,6 +13,8 @@
 // one at a time through 5 to 9 shared arrays, 12 sweeps and 12 barriers (FP64 p = 4 on 64^3 cells:
 // k(T) from its fields 0.91 -> 0.50 ms, deformed 0.95 -> 0.66 ms; FP32 p = 6 constant law on 45^3
 // cells 0.49 -> 0.28 ms, k(T) deformed 0.74 -> 0.47 ms). Shared memory and the barriers bound it.
+// FP32 p = 4 on deformed meshes, against register planes: 48^3 cells constant law 182 -> 162 us, k(T)
+// 254 -> 209 us; 30^3 liquid-solid 172 -> 65 us, three-phase fields 120 -> 59 us.
 // A thread rewrites only the lines it has read, so a batch needs no barrier before the next one.
 // z-lines are gathered and scattered with the lanes along x, so rows of nodes are contiguous.
 #pragma once
@@ -233,7 +235,7 @@ __global__ void __launch_bounds__(block_threads(n), (ln_min_blocks<n, T, GEO, LA
         asm volatile("prefetch.global.L2 [%0];" ::"l"(a.src + nb));
         asm volatile("prefetch.global.L2 [%0];" ::"l"(a.src + nb + n - 1));
         if (TDEP) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.Tl + nb));
-        constexpr int nf = LAW == 4 || LAW == 5 ? 5 : (LAW == 7 ? 4 : 0);
+        constexpr int nf = LAW == 4 || LAW == 5 ? 5 : (LAW == 6 ? 8 : (LAW == 7 ? 4 : 0));
         if constexpr (nf > 0) {
           const char *f = reinterpret_cast<const char *>(a.cf + next * nf * n3);
           for (int off = line * 128; off < nf * n3 * (int)sizeof(T); off += n2 * 128)
@@ -311,6 +313,14 @@ __global__ void __launch_bounds__(block_threads(n), (ln_min_blocks<n, T, GEO, LA
         f0 = kk * ux;
         f1 = kk * uy;
         f2 = kk * uz;
+      } else if constexpr (LAW == 6) {  // c u + rho_cp b.grad(u), flux k grad(u) + dk grad(T_lin) u
+        const T *cf = a.cf + cc * 8 * n3 + q0 + i;
+        const T kk = __ldg(cf + n3);
+        val = __ldg(cf) * uu + __ldg(cf + 2 * n3) * ux + __ldg(cf + 3 * n3) * uy +
+              __ldg(cf + 4 * n3) * uz;
+        f0 = kk * ux + __ldg(cf + 5 * n3) * uu;
+        f1 = kk * uy + __ldg(cf + 6 * n3) * uu;
+        f2 = kk * uz + __ldg(cf + 7 * n3) * uu;
       } else if constexpr (LAW == 7) {
         const T *cf = a.cf + cc * 4 * n3 + q0 + i;
         const T kk = __ldg(cf);

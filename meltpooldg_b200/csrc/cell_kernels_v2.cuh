@@ -341,8 +341,7 @@ __device__ __forceinline__ void load_map(const MeshDims &d, const double *__rest
 // warps, 0.96 ms against 0.52 ms with 128 registers, 16 warps, on 128^3 cells); a tighter bound
 // spills (0.56 ms at 20 warps; the FP64 k(T) tangent 1.71 ms at 12 warps, 1.36 ms at 8). Laws and
 // geometries that load per-point rows want more registers for the loads in flight (FP32 p = 3
-// deformed constant law on 96^3 cells: 0.36 ms at 12 warps, 0.40 ms at 16; p = 4 deformed k(T)
-// on 64^3 cells: 0.57 ms at 8 warps, 1.40 ms at 10 with spills).
+// deformed constant law on 96^3 cells: 0.36 ms at 12 warps, 0.40 ms at 16).
 template <int n, typename T, int GEO, int LAW> constexpr int v2_min_blocks()
 {
   constexpr bool rows = GEO != 0 || (LAW != 0 && LAW != 3);

@@ -82,9 +82,15 @@ struct DegreeOps {
   // the operator alone also with the constant law on a uniform box up to p = 5, which spills but
   // needs no per-point data (FP64 p = 4 on 64^3 cells 0.30 against 0.42 ms on lines, p = 5 on 53^3
   // 0.43 against 0.50 ms; FP32 p = 5 0.23 against 0.26 ms)
+  // ... and not in FP32 at p = 4 on a deformed mesh, except for the operators that exist on planes
+  // only (conductivity, LAW 3 and 8): a plane's rows of 5 values have no vector load and lie 100
+  // bytes apart from lane to lane, a line's do not (planes against lines: constant law on 48^3 cells
+  // 182, 162 us, on 6^3 11.2, 9.2; k(T) on 48^3 254, 209; liquid-solid on 30^3 172, 65, gas-liquid
+  // 91, 51)
   template <typename T, int GEO, int LAW>
   static constexpr bool vmult_v2()
   {
+    if (sizeof(T) == 4 && n == 5 && GEO == 1 && LAW != 3 && LAW != 8) return false;
     return use_v2<T, LAW>() || (GEO == 0 && LAW == 0 && n <= 6);
   }
 
