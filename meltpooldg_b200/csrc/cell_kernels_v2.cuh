@@ -301,11 +301,12 @@ __device__ __forceinline__ void mask_column(const ColumnMask &cm, T (&Q)[n][n])
 // evaluation (~55 operations a point, on FP64 units that the loads leave idle) is shorter than
 // reading 56 bytes a point: constant law p = 2 on 96^3 cells 0.36 -> 0.29 ms, p = 3 on 133^3 cells
 // 2.40 -> 1.87 ms, k(T) tangent p = 3 on 64^3 cells 0.54 -> 0.31 ms; at p = 1 a cell has as many
-// vertices as nodes and it is not (0.36 -> 0.40 ms on 160^3). FP32 keeps the stored factors, which
-// are rounded from FP64 ones.
-template <int n, typename T, int GEO> constexpr int v2_geometry()
+// vertices as nodes and it is not (0.36 -> 0.40 ms on 160^3), and the liquid-solid law at p = 3 has
+// no registers left for it (40^3 cells 183 us stored, 209 us evaluated). FP32 keeps the stored
+// factors, which are rounded from FP64 ones.
+template <int n, typename T, int GEO, int LAW> constexpr int v2_geometry()
 {
-  return GEO == 1 && sizeof(T) == 8 && n >= 3 ? 2 : GEO;
+  return GEO == 1 && sizeof(T) == 8 && n >= 3 && !(n == 4 && LAW == 2) ? 2 : GEO;
 }
 
 // The trilinear map of a cell on the plane zeta = const of its unit cube,

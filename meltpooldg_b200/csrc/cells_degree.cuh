@@ -121,7 +121,7 @@ struct DegreeOps {
   {
     static ResidentBlocks cache2;
     // deformed FP64: the geometry from the cell's vertices (p >= 2) instead of the stored one
-    constexpr int G = v2_geometry<n, T, GEO>();
+    constexpr int G = v2_geometry<n, T, GEO, LAW>();
     auto k2 = k_vmult2<n, T, G, LAW>;
     const size_t smem2 = v2_smem<n, T, LAW, G>();
     const bool dependent = v2_dependent<T>() && a.dependent;
