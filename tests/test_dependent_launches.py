@@ -1,5 +1,5 @@
-"""Kernels launched as programmatic dependents (launch.cuh) read what the iteration writes by coherent
-loads: they are resident while their predecessors still write it, and a non-coherent load (__ldg, or
+"""Kernels launched as programmatic dependents (launch.cuh) read what the iteration writes by
+coherent loads: they are resident while their predecessors still write it, and a non-coherent load (__ldg, or
 a const __restrict__ pointer) is defined only for data that nobody writes while the kernel lives.
 Read from the sources, since a violation need not show in a result."""
 import os
@@ -19,8 +19,12 @@ def dependent_kernels(src):
     for f, text in src.items():
         if f == "launch.cuh":
             continue
-        for m in re.finditer(r"launch_dependent\(\s*(\w+)", text):
-            name = m.group(1)
+        # directly, or by launch_persistent with its `dependent` argument
+        launches = r"launch_dependent\(\s*(\w+)|launch_persistent\(\w+,\s*(\w+)[^;]*?\bdependent\b"
+        for m in re.finditer(launches, text):
+            name = m.group(1) or m.group(2)
+            if name == "kernel":  # launch_persistent itself
+                continue
             if not name.startswith("k_"):  # a local: auto k = k_name<...>
                 name = re.findall(r"auto %s = (k_\w+)" % name, text[:m.start()])[-1]
             names.add(name)
