@@ -15,8 +15,8 @@ field plus the convective term of a velocity field), whose per-point coefficient
 gas): where the register-resident kernel exists (p <= 3 FP64, p <= 4 FP32) its 8
 tangent coefficients per point are built once per linearisation (reported as
 setup_ms, the first application minus a steady one) and the application reads src,
-dst and the coefficients; elsewhere the line-per-thread kernel reads src, dst, T_lin,
-T_old and 5 field values per point.
+dst and the coefficients; elsewhere the line kernel reads src, dst, T_lin, T_old and
+5 field values per point.
 """
 from __future__ import annotations
 

@@ -13,8 +13,8 @@
 // one at a time through 5 to 9 shared arrays, 12 sweeps and 12 barriers (FP64 p = 4 on 64^3 cells:
 // k(T) from its fields 0.91 -> 0.50 ms, deformed 0.95 -> 0.66 ms; FP32 p = 6 constant law on 45^3
 // cells 0.49 -> 0.28 ms, k(T) deformed 0.74 -> 0.47 ms). Shared memory and the barriers bound it.
-// FP32 p = 4 on deformed meshes, against register planes: 48^3 cells constant law 182 -> 162 us, k(T)
-// 254 -> 209 us; 30^3 liquid-solid 172 -> 65 us, three-phase fields 120 -> 59 us.
+// FP32 p = 4 on deformed meshes, against register planes: 48^3 cells constant law 182 -> 162 us,
+// k(T) 254 -> 209 us; 30^3 liquid-solid 172 -> 65 us, three-phase fields 120 -> 59 us.
 // A thread rewrites only the lines it has read, so a batch needs no barrier before the next one.
 // z-lines are gathered and scattered with the lanes along x, so rows of nodes are contiguous.
 #pragma once

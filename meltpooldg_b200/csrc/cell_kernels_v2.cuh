@@ -1,4 +1,5 @@
-// Register-resident cell kernel for the operator application (n = p + 1 <= 5).
+// Register-resident cell kernel for the operator application (n = p + 1 <= 4 in FP64, <= 5 in FP32;
+// the constant law on a uniform box n <= 6).
 //
 // Layout: every cell gets n threads of one warp (32/n cells per warp); thread t
 // holds one 2D plane of the cell's n^3 tensor in registers:

@@ -72,7 +72,7 @@ struct DegreeOps {
     cudaMemcpyToSymbol(c_w_f, wf, sizeof(float) * kWTabSize);
   }
 
-  // register-resident kernel where a cell's planes fit the register file; the three-phase /
+  // register-plane kernels where a cell's planes fit the register file; the three-phase /
   // transport law with temperature dependence (LAW 5) runs the line kernel
   template <typename T, int LAW = 0>
   static constexpr bool use_v2()

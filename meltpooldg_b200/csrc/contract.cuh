@@ -1,4 +1,4 @@
-// The 1D contraction of the cell kernels: one line of n values with an n x n matrix of fe_tables.hpp.
+// The 1D contraction of the cell kernels: a line of n values with an n x n matrix of fe_tables.hpp.
 // No CUDA header is needed, so that a host compiler can build it (with __device__ and
 // __forceinline__ defined) and its rounding can be tested on the CPU.
 #pragma once
@@ -24,12 +24,12 @@ template <typename T> __device__ __forceinline__ T ctab(int i);
 //   n = 4, 6 in FP64: E accumulates onto O and the mirror image takes 2 O off again, 2 h + 1
 //     operations, rounded h and h + 1 times (the operator's error 0.91-1.05 of separate parts').
 //   Else separate parts. O accumulated onto E rounds 2 h times at E's size: FP32 in as many
-//     operations at n = 4, 5 and more at 6, 7, with 1.10-1.17 (n = 4), 1.04-1.09 (5), 1.14-1.29 (6, 7)
-//     times the error; FP64 with twice E taken off for the mirror image 1.02-1.19 times.
+//     operations at n = 4, 5 and more at 6, 7, with 1.10-1.17 (n = 4), 1.04-1.09 (5), 1.14-1.29
+//     (6, 7) times the error; FP64 with twice E taken off for the mirror image 1.02-1.19 times.
 // (Emulated operator on sine products, a Gaussian of radius 0.05 and a temperature field; on random
-// operands, where E and O are alike, all forms are within 8 %.) On a B200 the FP64 forms take 1.33 ms
-// for the k(T) tangent on 128^3 cells of FE_Q(3) (with twice E 1.41), 375 us for FE_Q(5) on 53 x 49 x
-// 51 (416), 226 us for FE_Q(6) on 33^3 (218), 158 us for FE_Q(1) on 150^3 (155).
+// operands, where E and O are alike, all forms are within 8 %.) On a B200 the FP64 forms take
+// 1.33 ms for the k(T) tangent on 128^3 cells of FE_Q(3) (with twice E 1.41), 375 us for FE_Q(5) on
+// 53 x 49 x 51 (416), 226 us for FE_Q(6) on 33^3 (218), 158 us for FE_Q(1) on 150^3 (155).
 template <int n, int kind, bool add, typename T>
 __device__ __forceinline__ void contract_row(const T (&x)[n], T (&y)[n])
 {

@@ -7,8 +7,8 @@
 //
 // Such a kernel reads the vectors that the iteration writes by coherent loads: load_live, or plain
 // loads through pointers without __restrict__. It is resident while its predecessors still write
-// them, and a non-coherent load (__ldg, or what the compiler makes of const __restrict__) is defined
-// only for data that no one writes while the kernel lives; it may also be moved above
+// them, and a non-coherent load (__ldg, or what the compiler makes of const __restrict__) is
+// defined only for data that no one writes while the kernel lives; it may also be moved above
 // wait_for_predecessor. What stays fixed during the solve (the diagonal, coefficients, geometry,
 // indices) is read either way.
 #pragma once

@@ -126,7 +126,8 @@ struct mpdg_heat {
   double *tf = nullptr;
   float *tf_f = nullptr;
   bool tf_dirty = true, tf_f_dirty = true;
-  // tangent fields of the linear-k law at the linearisation point (4 per point, LAW 7)
+  // tangent fields of the linear-k law at the linearisation point (LAW 7): 2 per point on register planes,
+  // 4 for the line kernel
   double *tk = nullptr;
   bool tk_dirty = true;
   // GMRES basis (m + 1 vectors) and small device buffers
@@ -496,8 +497,9 @@ __global__ void k_distribute(DirArgs a, int face, double *u)
 
 // The same loop with kChunk values a thread and round, VT apart, whose loads are all issued before
 // the first use: one value a round leaves too few bytes in flight for HBM (the FP32 Chebyshev step
-// 0.322 -> 0.298 ms, the last one 0.68 -> 0.42, the CG update 0.73 -> 0.63 ms at 57 M DoFs). Scalar accesses: the vectors may
-// start at any element. Launched with chunk_grid, the blocks that are resident at once.
+// 0.322 -> 0.298 ms, the last one 0.68 -> 0.42, the CG update 0.73 -> 0.63 ms at 57 M DoFs). Scalar
+// accesses: the vectors may start at any element. Launched with chunk_grid, the blocks that are
+// resident at once.
 constexpr int kChunk = 4, kChunkBlocks = 4;  // (4 blocks of VT threads per SM: 64 registers)
 #define CHUNK_STRIDE(i0, N)                                                            \
   for (int64_t i0 = blockIdx.x * (int64_t)(VT * kChunk) + threadIdx.x; i0 < (N);       \
@@ -802,9 +804,9 @@ __global__ void k_cgm_init(int64_t N, const double *__restrict__ b, double *r, d
 // Chebyshev step: d = c1 d + c2 D32 (r32 - Ax32) ; x32 += d ; Ax32 = 0
 // (x in xr's cell rows instead of x32 with ROWS)
 template <bool ROWS>
-__global__ void __launch_bounds__(VT, kChunkBlocks) k_cheb_step(int64_t N, const float *__restrict__ r32, float *x32, float *d32,
-                            float *Ax32, const float *__restrict__ D32, float c1, float c2,
-                            const SolverState *st, CellRows xr)
+__global__ void __launch_bounds__(VT, kChunkBlocks)
+  k_cheb_step(int64_t N, const float *__restrict__ r32, float *x32, float *d32, float *Ax32,
+              const float *__restrict__ D32, float c1, float c2, const SolverState *st, CellRows xr)
 {
   if (st->done) return;
   CHUNK_STRIDE(i0, N)
@@ -835,10 +837,10 @@ __global__ void __launch_bounds__(VT, kChunkBlocks) k_cheb_step(int64_t N, const
 // flexible (Polak-Ribiere) beta = z.(r - r_old) / rz_old = -alpha z.Ap / rz_old
 // (x in xr's cell rows instead of x32 with ROWS)
 template <bool ROWS>
-__global__ void __launch_bounds__(VT, kChunkBlocks) k_cheb_last(int64_t N, const float *__restrict__ r32, const float *__restrict__ x32,
-                            const float *__restrict__ d32, float *Ax32,
-                            const float *__restrict__ D32, float c1, float c2,
-                            const double *__restrict__ r, const double *__restrict__ Ap, double *z,
+__global__ void __launch_bounds__(VT, kChunkBlocks)
+  k_cheb_last(int64_t N, const float *__restrict__ r32, const float *__restrict__ x32,
+              const float *__restrict__ d32, float *Ax32, const float *__restrict__ D32, float c1,
+              float c2, const double *__restrict__ r, const double *__restrict__ Ap, double *z,
                             SolverState *st, double *partials, unsigned *counter, CellRows xr)
 {
   if (st->done) return;
@@ -882,10 +884,11 @@ __global__ void __launch_bounds__(VT, kChunkBlocks) k_cheb_last(int64_t N, const
 
 // x += alpha p ; r -= alpha Ap ; rr ; r32 = r ; x32 = D32 r32 / theta ; d32 = x32
 template <bool ROWS>
-__global__ void __launch_bounds__(VT, kChunkBlocks) k_cgm_update_xr(int64_t N, double *x, double *r, const double *__restrict__ p,
-                                const double *__restrict__ Ap, float *r32, float *x32, float *d32,
-                                const float *__restrict__ D32, float inv_theta, SolverState *st,
-                                double *partials, unsigned *counter, CellRows xr)
+__global__ void __launch_bounds__(VT, kChunkBlocks)
+  k_cgm_update_xr(int64_t N, double *x, double *r, const double *__restrict__ p,
+                  const double *__restrict__ Ap, float *r32, float *x32, float *d32,
+                  const float *__restrict__ D32, float inv_theta, SolverState *st,
+                  double *partials, unsigned *counter, CellRows xr)
 {
   if (st->done) return;
   const double alpha = st->alpha;
@@ -923,8 +926,9 @@ __global__ void __launch_bounds__(VT, kChunkBlocks) k_cgm_update_xr(int64_t N, d
 }
 
 // p = z + beta p ; Ap = 0
-__global__ void __launch_bounds__(VT, kChunkBlocks) k_cgm_update_p(int64_t N, const double *__restrict__ z, double *p, double *Ap,
-                               const SolverState *st)
+__global__ void __launch_bounds__(VT, kChunkBlocks)
+  k_cgm_update_p(int64_t N, const double *__restrict__ z, double *p, double *Ap,
+                 const SolverState *st)
 {
   if (st->done) return;
   const double beta = st->beta;
@@ -2271,7 +2275,6 @@ static int mg_setup(mpdg_heat *h, const mpdg_solver_params *prm, bool picard)
   return MPDG_OK;
 }
 
-// coarse = R (fine_b - fine_Ax)
 static TransferArgs transfer_args(const MGLevel &f, const Dims3 &F, const Dims3 &C, int axis)
 {
   TransferArgs t;
@@ -2294,6 +2297,7 @@ static unsigned run_grid(const mpdg_heat *h, TransferArgs &t)
   while (t.run > 1 && across * ((t.n_coarse + t.run - 1) / t.run) < 2 * h->sm_count) t.run /= 2;
   return (unsigned)(across * ((t.n_coarse + t.run - 1) / t.run));
 }
+// coarse = R (fine_b - fine_Ax)
 static int mg_restrict(mpdg_heat *h, int l, const float *fine_Ax, const float *fine_b,
                        float *coarse)
 {
@@ -2354,14 +2358,14 @@ static int mg_prolong_add(mpdg_heat *h, int l, const float *coarse, float *fine,
 }
 
 template <bool ROWS>
-__global__ void __launch_bounds__(VT, kChunkBlocks) k_cheb_step(int64_t N, const float *__restrict__ r32, float *x32, float *d32,
-                            float *Ax32, const float *__restrict__ D32, float c1, float c2,
-                            const SolverState *st, CellRows xr);
+__global__ void __launch_bounds__(VT, kChunkBlocks)
+  k_cheb_step(int64_t N, const float *__restrict__ r32, float *x32, float *d32, float *Ax32,
+              const float *__restrict__ D32, float c1, float c2, const SolverState *st, CellRows xr);
 template <bool ROWS>
-__global__ void __launch_bounds__(VT, kChunkBlocks) k_cheb_last(int64_t N, const float *__restrict__ r32, const float *__restrict__ x32,
-                            const float *__restrict__ d32, float *Ax32,
-                            const float *__restrict__ D32, float c1, float c2,
-                            const double *__restrict__ r, const double *__restrict__ Ap, double *z,
+__global__ void __launch_bounds__(VT, kChunkBlocks)
+  k_cheb_last(int64_t N, const float *__restrict__ r32, const float *__restrict__ x32,
+              const float *__restrict__ d32, float *Ax32, const float *__restrict__ D32, float c1,
+              float c2, const double *__restrict__ r, const double *__restrict__ Ap, double *z,
                             SolverState *st, double *partials, unsigned *counter, CellRows xr);
 
 // one V-cycle on the FP32 residual in level 0's b (= r32), whose first smoothing step
