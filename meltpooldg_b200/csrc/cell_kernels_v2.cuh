@@ -1006,7 +1006,7 @@ __device__ __forceinline__ void add_outer(int q, const double (&x)[n], double (&
 //   Y_Q = P_y P_x Gzz      Y_R = P_y (R_x Gxz + P_x Bz) + R_y P_x Gyz
 //   W = P_z Y_P + Q_z Y_Q + R_z Y_R
 // so that no coefficient plane is kept (k_diag keeps ten in shared memory and takes 28 barriers a
-// batch; the inverse diagonal on 64^3 cells of FE_Q(3) k(T) 673 -> 183 us, deformed 768 -> 366).
+// batch; the inverse diagonal on 64^3 cells of FE_Q(3) k(T) 673 -> 208 us, deformed 768 -> 394).
 template <int n, int GEO, int LAW>
 __global__ void __launch_bounds__(32 * kV2Warps, 4) k_diag2(CellArgs<double> a)
 {
